@@ -91,6 +91,7 @@ void BatchSlot::ensure(int want_cap, int want_ln, int n_jobs, size_t n_offsets, 
       Q.sh_d = (float4 *)alloc(c * 16 * want_ln);
       Q.sh_c = (float4 *)alloc(c * 16 * want_ln);
       Q.sh_vis = (uint8_t *)alloc(c * want_ln);
+      Q.sh_list = (uint32_t *)alloc(c * 4 * want_ln);
       Q.counts = (int *)alloc(64);
       Q.stats = (unsigned long long *)alloc(64);
       Q.err = (int *)alloc(16);

@@ -1532,9 +1532,6 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   V.n_nodes = (int)out.nodes.size();
   V.n_prims = n_prims;
   V.trav_cap = trav_cap > 0 ? trav_cap : PT_TRAVERSAL_CAP;
-  // a node visit pushes at most 3 entries per level, plus a moving object's
-  // frame marker; 2 entries to spare
-  V.stack_entries = std::min(PT_STACK, 3 * out.max_depth + 4);
   for (int c = 0; c < 3; ++c) V.bg[c] = d->bg_color[c];
   if (d->env) {
     V.env.texels = up(tex);
@@ -1619,7 +1616,8 @@ Context::Context(int dev) : device(dev) {
   cfg.sort_by_material = 1;
   cfg.family_mask = 0x7f;
   const char *cap = std::getenv("PT_WAVE_PATHS");
-  wave_cap = cap ? std::max(1024, std::atoi(cap)) : (1 << 24);
+  // at most 2^28 - 1 paths: the shadow-ray list keeps a vertex slot in 28 bits
+  wave_cap = cap ? std::min(std::max(1024, std::atoi(cap)), (1 << PT_LIST_SHIFT) - 1) : (1 << 24);
   if (cap) batch_wave_cap = wave_cap;  // batched waves of the same size (tests of many-wave renders)
   // bound on one ray's traversal steps (scenes uploaded by this context);
   // exceeding it sets the device error flag, reported as PT_ERR_DEVICE
@@ -1635,8 +1633,9 @@ Context::Context(int dev) : device(dev) {
   cfg.pair_from_bounce = 0;
   const char *pfb = std::getenv("PT_PAIR_FROM_BOUNCE");
   if (pfb) cfg.pair_from_bounce = std::max(0, std::atoi(pfb));
-  cuda_check(cudaMalloc(&d_err, sizeof(int)), "cudaMalloc(err)");
-  cuda_check(cudaMemsetAsync(d_err, 0, sizeof(int), stream), "memset err");
+  cuda_check(cudaMalloc(&d_err, 2 * sizeof(int)), "cudaMalloc(err)");
+  d_fetch = d_err + 1;
+  cuda_check(cudaMemsetAsync(d_err, 0, 2 * sizeof(int), stream), "memset err");
   cuda_check(cudaStreamSynchronize(stream), "context init");
 }
 
@@ -1689,6 +1688,7 @@ static void alloc_queues(Queues &Q, std::vector<void *> &mem, int cap, int ln, i
   Q.sh_d = (float4 *)alloc(c * 16 * ln);
   Q.sh_c = (float4 *)alloc(c * 16 * ln);
   Q.sh_vis = (uint8_t *)alloc(c * ln);
+  Q.sh_list = (uint32_t *)alloc(c * 4 * ln);
   Q.counts = (int *)alloc(64);
   Q.stats = (unsigned long long *)alloc(64);
   Q.sort_key = (int *)alloc(c * 4);
@@ -2353,7 +2353,7 @@ static int trace_common(void *ctx, int32_t scene_id, bool any, const float *rays
     uint8_t *docc = (uint8_t *)(buf + nn * 44);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
     if (any) cuda_check(cudaMemcpyAsync(dtm, tmaxs, nn * 4, cudaMemcpyHostToDevice, c->stream), "h2d tmax");
-    launch_trace_test(S->view, any, dr, dtm, n, tmin, tmax, dt, dp, duv, docc, c->d_err, c->stream);
+    launch_trace_test(S->view, any, dr, dtm, n, tmin, tmax, dt, dp, duv, docc, c->d_fetch, c->d_err, c->stream);
     cuda_check(cudaGetLastError(), "trace launch");
     if (any) {
       cuda_check(cudaMemcpyAsync(occ, docc, nn, cudaMemcpyDeviceToHost, c->stream), "d2h");
@@ -2401,7 +2401,7 @@ int pt_intersect(void *ctx, int32_t scene_id, const float *rays, int32_t n, floa
     float *dn = (float *)(buf + nn * 44);
     uint8_t *df = (uint8_t *)(buf + nn * 56);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
-    launch_intersect(S->view, dr, n, tmin, tmax, dt, dp, dpos, dn, df, c->d_err, c->stream);
+    launch_intersect(S->view, dr, n, tmin, tmax, dt, dp, dpos, dn, df, c->d_fetch, c->d_err, c->stream);
     cuda_check(cudaGetLastError(), "intersect launch");
     cuda_check(cudaMemcpyAsync(t, dt, nn * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
     cuda_check(cudaMemcpyAsync(prim, dp, nn * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");

@@ -134,7 +134,8 @@ struct Context {
   int offsets_cap = 0;
   void *d_scratch = nullptr;
   size_t scratch_cap = 0;
-  int *d_err = nullptr;
+  int *d_err = nullptr;    // device error flag
+  int *d_fetch = nullptr;  // fetch counter of the ray-query kernels (behind d_err)
   Profiler prof;
   Batch batch;
   int batch_wave_cap = 1 << 22;  // paths per wave of each batched job

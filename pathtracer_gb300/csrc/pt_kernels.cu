@@ -68,27 +68,35 @@ void launch_path_samples(const DeviceJob &J, long long first, int n, int dims, i
   k_path_samples<<<grid_for(n, 128, 152 * 8), 128, 0, st>>>(J, first, n, dims, bounces, LN, pix, dv, lo);
 }
 
+// The batch ray queries: closest hits or occlusion of n given rays, *fetch = 0
+// at the start.
 template <bool ANY>
-__global__ void __launch_bounds__(128) k_trace_test(SceneView S, const float *rays, const float *tmaxs,
-                                                    int n, float tmin, float tmax, float *t_out,
-                                                    int *prim_out, float *uv_out, uint8_t *occ,
-                                                    int *err) {
-  extern __shared__ int32_t stack[];  // S.stack_entries x 128
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    V3 o = v3(rays[6 * i], rays[6 * i + 1], rays[6 * i + 2]);
-    V3 d = v3(rays[6 * i + 3], rays[6 * i + 4], rays[6 * i + 5]);
-    HitRec h;
-    float tm = ANY ? tmaxs[i] : tmax;
-    bool r = traverse<ANY>(S, o, d, tmin, tm, h, stack + threadIdx.x, blockDim.x, err);
-    if (ANY) {
-      occ[i] = r ? 1 : 0;
-    } else {
-      t_out[i] = r ? h.t : FLT_MAX;
-      prim_out[i] = r ? h.prim : -1;
-      uv_out[2 * i] = h.u;
-      uv_out[2 * i + 1] = h.v;
-    }
-  }
+__global__ void __launch_bounds__(128) k_trace_test(SceneView S, const float *rays, const float *tmaxs, int n,
+                                                    float tmin, float tmax, float *t_out, int *prim_out, float *uv_out,
+                                                    uint8_t *occ, int *fetch, int *err) {
+  extern __shared__ __align__(16) char smem[];  // trace_smem
+  int i = 0;
+  trace_rays<ANY ? TRACE_ANY : TRACE_CLOSEST, true>(
+      S, n, fetch, ANY ? PT_FETCH_IDLE_SHADOW : PT_FETCH_IDLE, err, smem,
+      [&](int r, V3 &o, V3 &d, float &t0, float &t1, float &, bool &) {
+        i = r;
+        const float *p = rays + 6 * (size_t)r;
+        o = v3(p[0], p[1], p[2]);
+        d = v3(p[3], p[4], p[5]);
+        t0 = tmin;
+        t1 = ANY ? tmaxs[r] : tmax;
+        return true;
+      },
+      [&](bool found, const HitRec &h) {
+        if (ANY) {
+          occ[i] = found ? 1 : 0;
+        } else {
+          t_out[i] = found ? h.t : FLT_MAX;
+          prim_out[i] = found ? h.prim : -1;
+          uv_out[2 * (size_t)i] = found ? h.u : 0.f;
+          uv_out[2 * (size_t)i + 1] = found ? h.v : 0.f;
+        }
+      });
 }
 
 // Hittable::intersect's HitRecord (base/primitive.hpp:30-79) at the closest
@@ -97,33 +105,43 @@ __global__ void __launch_bounds__(128) k_trace_test(SceneView S, const float *ra
 // toggled) -- what surface_at gives the shade stage.
 __global__ void __launch_bounds__(128) k_intersect(SceneView S, const float *rays, int n, float tmin, float tmax,
                                                    float *t_out, int *prim_out, float *pos, float *nrm,
-                                                   uint8_t *front, int *err) {
-  extern __shared__ int32_t stack[];  // S.stack_entries x 128
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const V3 o = v3(rays[6 * i], rays[6 * i + 1], rays[6 * i + 2]);
-    const V3 d = v3(rays[6 * i + 3], rays[6 * i + 4], rays[6 * i + 5]);
-    HitRec h;
-    const bool r = traverse<false>(S, o, d, tmin, tmax, h, stack + threadIdx.x, blockDim.x, err);
-    Surf sf;
-    sf.p = sf.n = v3(0.f);
-    sf.front = false;
-    if (r) sf = surface_at(S, o, d, h, 0.f);
-    t_out[i] = r ? h.t : FLT_MAX;
-    prim_out[i] = r ? h.prim : -1;
-    pos[3 * i] = sf.p.x;
-    pos[3 * i + 1] = sf.p.y;
-    pos[3 * i + 2] = sf.p.z;
-    nrm[3 * i] = sf.n.x;
-    nrm[3 * i + 1] = sf.n.y;
-    nrm[3 * i + 2] = sf.n.z;
-    front[i] = (r && sf.front) ? 1 : 0;
-  }
+                                                   uint8_t *front, int *fetch, int *err) {
+  extern __shared__ __align__(16) char smem[];  // trace_smem
+  int i = 0;
+  trace_rays<TRACE_CLOSEST, true>(
+      S, n, fetch, PT_FETCH_IDLE, err, smem,
+      [&](int r, V3 &o, V3 &d, float &t0, float &t1, float &, bool &) {
+        i = r;
+        const float *p = rays + 6 * (size_t)r;
+        o = v3(p[0], p[1], p[2]);
+        d = v3(p[3], p[4], p[5]);
+        t0 = tmin;
+        t1 = tmax;
+        return true;
+      },
+      [&](bool found, const HitRec &h) {
+        const float *p = rays + 6 * (size_t)i;
+        Surf sf;
+        sf.p = sf.n = v3(0.f);
+        sf.front = false;
+        if (found) sf = surface_at(S, v3(p[0], p[1], p[2]), v3(p[3], p[4], p[5]), h, 0.f);
+        t_out[i] = found ? h.t : FLT_MAX;
+        prim_out[i] = found ? h.prim : -1;
+        pos[3 * (size_t)i] = sf.p.x;
+        pos[3 * (size_t)i + 1] = sf.p.y;
+        pos[3 * (size_t)i + 2] = sf.p.z;
+        nrm[3 * (size_t)i] = sf.n.x;
+        nrm[3 * (size_t)i + 1] = sf.n.y;
+        nrm[3 * (size_t)i + 2] = sf.n.z;
+        front[i] = (found && sf.front) ? 1 : 0;
+      });
 }
 
 void launch_intersect(const SceneView &S, const float *rays, int n, float tmin, float tmax, float *t, int *prim,
-                      float *pos, float *nrm, uint8_t *front, int *err, cudaStream_t st) {
-  k_intersect<<<grid_for(n, 128, 152 * 8), 128, stack_bytes(S, 128), st>>>(S, rays, n, tmin, tmax, t, prim, pos, nrm,
-                                                                         front, err);
+                      float *pos, float *nrm, uint8_t *front, int *fetch, int *err, cudaStream_t st) {
+  cudaMemsetAsync(fetch, 0, sizeof(int), st);
+  k_intersect<<<grid_for(n, 128, 152 * 7), 128, trace_smem(S, 128), st>>>(S, rays, n, tmin, tmax, t, prim, pos, nrm,
+                                                                         front, fetch, err);
 }
 
 // The Light methods of one light of a resident scene at n (u, v, x) items:
@@ -265,9 +283,9 @@ __global__ void k_sort_scatter(Queues Q, int qsel) {
 // k_trace_shadow, k_shadow_resolve, k_film: their bodies are in pt_wave.cuh
 // (trace_shadow_body, shadow_resolve_body, film_body).
 template <bool CURVES>
-__global__ void __launch_bounds__(128) k_trace_shadow(SceneView S, Queues Q, int LN) {
-  extern __shared__ int32_t stack[];  // S.stack_entries x 128
-  trace_shadow_body<CURVES>(S, Q, LN, stack);
+__global__ void __launch_bounds__(128) k_trace_shadow(SceneView S, Queues Q) {
+  extern __shared__ __align__(16) char smem[];  // trace_smem
+  trace_shadow_body<CURVES>(S, Q, smem);
 }
 __global__ void k_shadow_resolve(Queues Q, int LN) { shadow_resolve_body(Q, LN); }
 __global__ void k_film(DeviceJob J, Queues Q, long long g0, int n, long long slot0, float *film) {
@@ -362,13 +380,15 @@ void launch_sampler_eval(int strategy, const uint16_t *perm, uint32_t first, int
 }
 
 void launch_trace_test(const SceneView &S, bool any, const float *rays, const float *tmaxs, int n,
-                       float tmin, float tmax, float *t, int *prim, float *uv, uint8_t *occ, int *err,
+                       float tmin, float tmax, float *t, int *prim, float *uv, uint8_t *occ, int *fetch, int *err,
                        cudaStream_t st) {
-  int g = grid_for(n, 128, 152 * 8);
+  const int g = grid_for(n, 128, 152 * 7);
+  cudaMemsetAsync(fetch, 0, sizeof(int), st);
   if (any)
-    k_trace_test<true><<<g, 128, stack_bytes(S, 128), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, err);
+    k_trace_test<true><<<g, 128, trace_smem(S, 128, true), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, fetch,
+                                                                 err);
   else
-    k_trace_test<false><<<g, 128, stack_bytes(S, 128), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, err);
+    k_trace_test<false><<<g, 128, trace_smem(S, 128), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, fetch, err);
 }
 
 void launch_bsdf_eval(const MatRec *m, int n, const float *wo, const float *wi, const float *nrm,
@@ -408,9 +428,9 @@ void launch_sort(const SceneView &S, const Queues &Q, int qsel, const LaunchCfg 
 
 void launch_shadow(const SceneView &S, const Queues &Q, int LN, const LaunchCfg &cfg, cudaStream_t st) {
   if (S.curves)
-    k_trace_shadow<true><<<cfg.trace_blocks, 128, stack_bytes(S, 128), st>>>(S, Q, LN);
+    k_trace_shadow<true><<<cfg.trace_blocks, 128, trace_smem(S, 128, true), st>>>(S, Q);
   else
-    k_trace_shadow<false><<<cfg.trace_blocks, 128, stack_bytes(S, 128), st>>>(S, Q, LN);
+    k_trace_shadow<false><<<cfg.trace_blocks, 128, trace_smem(S, 128, true), st>>>(S, Q);
   k_shadow_resolve<<<cfg.max_blocks_simple, 256, 0, st>>>(Q, LN);
 }
 void launch_shadow_resolve(const Queues &Q, int LN, const LaunchCfg &cfg, cudaStream_t st) {
@@ -448,8 +468,9 @@ void kernel_attributes(KernelInfo *info) {
   cudaFuncGetAttributes(&a, k_shade<-1, false>);
   info->shade_regs = a.numRegs;
   int nb = 0;
-  // occupancy at the largest stack (the grids must fit every scene)
-  const size_t smax = (size_t)PT_STACK * 128 * sizeof(int32_t);
+  SceneView any_scene{};  // occupancy at the largest shared memory (the grids must fit every scene)
+  any_scene.has_motion = 1;
+  const size_t smax = trace_smem(any_scene, 128);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_closest<false, false>, 128, smax);
   info->trace_blocks_per_sm = nb;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade<-1, false>, 128, 0);

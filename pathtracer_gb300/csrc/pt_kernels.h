@@ -16,6 +16,8 @@
 #define PT_KEY_MEDIUM 9
 #define PT_FAM_MISC 7
 #define PT_HIT_MEDIUM (-2)
+// Shadow-ray list entries: the vertex slot below, the light sample above.
+#define PT_LIST_SHIFT 28
 
 namespace pt {
 
@@ -41,10 +43,11 @@ struct Queues {
   float4 *ray_d[2];   //                     direction.xyz
   float4 *hit;        // HitQueue: t, prim (int bits), u, v
   float4 *sh_o;       // ShadowQueue: origin.xyz, path slot
-  float4 *sh_d;       // [light sample][cap]: direction.xyz, tmax (<0: none)
+  float4 *sh_d;       // [light sample][cap]: direction.xyz, tmax (contributing samples)
   float4 *sh_c;       // [light sample][cap]: unoccluded contribution
   uint8_t *sh_vis;    // [light sample][cap]: 1 = the shadow ray reached the light
-  int *counts;        // [0],[1] ray queues, [2] shadow queue, [3] [4] fetch counters
+  uint32_t *sh_list;  // the shadow rays to trace: vertex slot | light sample << PT_LIST_SHIFT
+  int *counts;        // [0],[1] ray queues, [2] shadow queue, [3] [4] fetch counters, [5] listed shadow rays
   unsigned long long *stats;  // [0] paths [1] segments [2] rays [3] shadow rays
   int *err;           // device error flag (stack overflow / iteration cap)
   int *job;           // [cap] merged waves: job index of the path in each slot
@@ -136,14 +139,14 @@ void upload_halton_tables(const HaltonTables &T, cudaStream_t st);
 void launch_light_eval(const SceneView &S, int light, int n, const float *uv, const float *x, const float *pdf_dir,
                        float *point, float *normal, float *dir, float *le, float *pdf, cudaStream_t st);
 void launch_intersect(const SceneView &S, const float *rays, int n, float tmin, float tmax, float *t, int *prim,
-                      float *pos, float *nrm, uint8_t *front, int *err, cudaStream_t st);
+                      float *pos, float *nrm, uint8_t *front, int *fetch, int *err, cudaStream_t st);
 void launch_path_samples(const DeviceJob &J, long long first, int n, int dims, int bounces, float *pix, float *dv,
                          float *lo, cudaStream_t st);
 void launch_sampler_eval(int strategy, const uint16_t *perm, uint32_t first, int n, int dims,
                          float *out, cudaStream_t st);
 void launch_trace_test(const SceneView &S, bool any, const float *rays, const float *tmaxs, int n,
                        float tmin, float tmax, float *t, int *prim, float *uv, uint8_t *occ,
-                       int *err, cudaStream_t st);
+                       int *fetch, int *err, cudaStream_t st);
 void launch_bsdf_eval(const MatRec *m, int n, const float *wo, const float *wi, const float *nrm,
                       const uint8_t *front, float *f, float *pdf, cudaStream_t st);
 void launch_bsdf_sample(const MatRec *m, int n, const float *wo, const float *nrm,

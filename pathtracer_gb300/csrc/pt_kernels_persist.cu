@@ -89,19 +89,19 @@ struct NoReset {
 // and spills), and reads the kernel's parameters in place (__grid_constant__).
 template <bool CURVES>
 __device__ __noinline__ void st_trace(const SceneView &S, const DeviceJob &none, const JobTable &T, const Queues &Q,
-                                      int qsel, int b, long long g0, int LN, int32_t *stack) {
+                                      int qsel, int b, long long g0, char *smem) {
   if (b > 0)
-    trace_pair_body<true, CURVES>(S, none, T, Q, qsel, b, g0, LN, stack);
+    trace_pair_body<true, CURVES>(S, none, T, Q, qsel, b, g0, smem);
   else
-    trace_closest_body<true, CURVES>(S, none, T, Q, qsel, b, g0, stack);
+    trace_closest_body<true, CURVES>(S, none, T, Q, qsel, b, g0, smem);
 }
 __device__ __noinline__ void st_shade(const SceneView &S, const DeviceJob &none, const JobTable &T, const Queues &Q,
                                       int qsel, int b, long long g0) {
   shade_body<-1, true>(S, none, T, Q, qsel, b, g0);
 }
 template <bool CURVES>
-__device__ __noinline__ void st_shadow(const SceneView &S, const Queues &Q, int LN, int32_t *stack) {
-  trace_shadow_body<CURVES>(S, Q, LN, stack);
+__device__ __noinline__ void st_shadow(const SceneView &S, const Queues &Q, char *smem) {
+  trace_shadow_body<CURVES>(S, Q, smem);
 }
 
 // The whole group: for each wave of `wave` paths over [0, total), camera ->
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
     k_group_persistent(const __grid_constant__ SceneView S, const __grid_constant__ JobTable T,
                        const __grid_constant__ Queues Q, float *const *films, long long total, int wave, int LN,
                        int bounces, GridBarrier *bar) {
-  extern __shared__ int32_t stack[];  // S.stack_entries x PT_PERSIST_THREADS
+  extern __shared__ __align__(16) char smem[];  // trace_smem
   __shared__ DeviceJob none;  // unused by merged waves (each path's job comes from T)
   if (threadIdx.x == 0) memset(&none, 0, sizeof none);
   __syncthreads();
@@ -120,21 +120,21 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
   for (long long g0 = 0; g0 < total; g0 += wave) {
     const int n = (int)min((long long)wave, total - g0);
     camera_body<true>(none, T, Q, g0, n);
-    if (!grid_sync(bar, [=] { cnt[1] = 0; cnt[2] = 0; cnt[3] = 0; cnt[4] = 0; })) return;
+    if (!grid_sync(bar, [=] { cnt[1] = 0; cnt[2] = 0; cnt[3] = 0; cnt[4] = 0; cnt[5] = 0; })) return;
     int qsel = 0;
     for (int b = 0; b < bounces; ++b) {
-      st_trace<CURVES>(S, none, T, Q, qsel, b, g0, LN, stack);
+      st_trace<CURVES>(S, none, T, Q, qsel, b, g0, smem);
       const int nq = qsel ^ 1;
       if (!grid_sync(bar, [=] { cnt[nq] = 0; cnt[4] = 0; })) return;
       if (b > 0) {
         shadow_resolve_body(Q, LN);
-        if (!grid_sync(bar, [=] { cnt[2] = 0; cnt[3] = 0; })) return;
+        if (!grid_sync(bar, [=] { cnt[2] = 0; cnt[3] = 0; cnt[5] = 0; })) return;
       }
       st_shade(S, none, T, Q, qsel, b, g0);
       if (!grid_sync(bar, NoReset())) return;
       qsel = nq;
     }
-    st_shadow<CURVES>(S, Q, LN, stack);
+    st_shadow<CURVES>(S, Q, smem);
     if (!grid_sync(bar, NoReset())) return;
     shadow_resolve_body(Q, LN);
     if (!grid_sync(bar, NoReset())) return;
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
 
 int persistent_grid(const SceneView &S, int num_sms) {
   int per = 0;
-  const size_t smem = stack_bytes(S, PT_PERSIST_THREADS);
+  const size_t smem = trace_smem(S, PT_PERSIST_THREADS);
   if (S.curves)
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_group_persistent<true>, PT_PERSIST_THREADS, smem);
   else
@@ -170,7 +170,7 @@ cudaError_t launch_group_persistent(const SceneView &S, const JobTable &T, const
   void *args[] = {&s, &t, &q, &f, &total, &wave, &LN, &bounces, &b};
   const void *fn = S.curves ? (const void *)k_group_persistent<true> : (const void *)k_group_persistent<false>;
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PT_PERSIST_THREADS), args,
-                                     stack_bytes(S, PT_PERSIST_THREADS), st);
+                                     trace_smem(S, PT_PERSIST_THREADS), st);
 }
 
 }  // namespace pt

@@ -2,9 +2,9 @@
 //
 // The BVH4 is collapsed from the reference's own binary trees (top level
 // BVHNode, bvh.hpp:46-102; per mesh MeshBVHNode, meshBVH.cpp:6-55), so the
-// leaves hold exactly the reference's leaf primitive sets.  Traversal is
-// near-to-far with a per-thread stack in SHARED memory (column per thread,
-// bank-conflict free).  Primitive tests restate the reference arithmetic
+// leaves hold exactly the reference's leaf primitive sets.  Closest-hit
+// traversal is near-to-far; the per-thread stacks are in SHARED memory
+// (column per thread, bank-conflict free).  Primitive tests restate the reference arithmetic
 // with rounded, never-fused operations so that hit distances match the
 // reference bit for bit:
 //   triangle  MeshBVHNode::hitTriangle  meshBVH.cpp:85-143
@@ -184,7 +184,6 @@ __device__ __forceinline__ Item load_item(const Item *items, int i) {
   return it;
 }
 
-// Tests one leaf; for ANY returns true on the first hit in [tmin, tmax].
 // Origin of a ray of time `time` in the frame of a primitive moving with
 // velocity v: o - v * time (rounded, never fused).
 __device__ __forceinline__ V3 moved_origin(const SceneView &S, uint32_t motion, V3 o, float time) {
@@ -192,32 +191,30 @@ __device__ __forceinline__ V3 moved_origin(const SceneView &S, uint32_t motion, 
   return v3(xsub(o.x, xmul(v.x, time)), xsub(o.y, xmul(v.y, time)), xsub(o.z, xmul(v.z, time)));
 }
 
-// Tests leaf item `idx` (a whole leaf is its items in order); for ANY
-// returns true on a hit in [tmin, tmax], for closest hit records the hit and
-// shrinks tmax (acceptance is inclusive: of equal-t items the later wins).
-// CURVES = false compiles the curve test out (curve items then never hit):
-// the closest-hit kernel of a scene without curves keeps 8 fewer registers.
-template <bool ANY, bool CURVES = true>
-__device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V3 d, V3 dn, float tmin,
-                                          float &tmax, HitRec &hit, float time) {
+// Tests leaf item `idx` against a ray (origin o in its current frame); a
+// hit in [tmin, tmax] fills `hit`.  dn points at the ray's normalised
+// direction (rectangles and spheres read it).  CURVES = false compiles the
+// curve test out (curve items then never hit).
+template <bool CURVES>
+__device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V3 d, const float4 *dn4, float tmin,
+                                          float tmax, HitRec &hit, float time) {
   Item it = load_item(S.items, idx);
   const int type = (int)f2u(it.b[3]);
   const uint32_t motion = f2u(it.c[3]);
   const V3 o = motion ? moved_origin(S, motion, o_w, time) : o_w;
   float t, u = 0.f, v = 0.f;
   bool h;
-  if (type == ITEM_TRI)
+  if (type == ITEM_TRI) {
     h = hit_triangle(it, o, d, tmin, tmax, t, u, v);
-  else if (type == ITEM_QUAD)
-    h = hit_quad(it, o, dn, tmin, tmax, t);
-  else if (type == ITEM_SPHERE)
-    h = hit_sphere(it, o, dn, tmin, tmax, t);
-  else if (CURVES)
+  } else if (CURVES && type == ITEM_CURVE) {
     h = hit_curve(S.curves + 4 * (size_t)f2u(it.a[0]), o, d, tmin, tmax, t, u, v);
-  else
+  } else if (type == ITEM_CURVE) {
     h = false;
-  if (h && !ANY) {
-    tmax = t;
+  } else {
+    const V3 dn = v3(dn4->x, dn4->y, dn4->z);
+    h = type == ITEM_QUAD ? hit_quad(it, o, dn, tmin, tmax, t) : hit_sphere(it, o, dn, tmin, tmax, t);
+  }
+  if (h) {
     hit.t = t;
     hit.prim = (int32_t)f2u(it.a[3]);
     hit.u = u;
@@ -226,24 +223,10 @@ __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V
   return h;
 }
 
-// Traversal state of one ray.  The walk is a sequence of node visits and
-// leaf tests (trav_step) so that a persistent warp can refill lanes whose
-// rays have finished while the others continue.
-struct TravRay {
-  V3 o, d, dn, inv, oi;  // o, oi: the current frame (world, or a moving object's)
-  V3 ow;                 // world origin
-  float tmin, tmax;
-  int32_t ref;   // next reference: node (>= 0, PT_INST_BIT: entering a moving
-                 // object), leaf (< 0), PT_FRAME_END or PT_REF_EMPTY
-  int sp;        // stack depth
-  int iters;
-  float time;    // motion blur: the ray's time
-  bool found;
-  HitRec hit;
-};
-
 __device__ __forceinline__ bool ref_is_node(int32_t r) { return r >= 0 || r == PT_FRAME_END; }
 __device__ __forceinline__ bool ref_is_leaf(int32_t r) { return r < 0 && r != PT_FRAME_END && r != PT_REF_EMPTY; }
+// References that change the ray's frame (moving objects).
+__device__ __forceinline__ bool ref_is_frame(int32_t r) { return r == PT_FRAME_END || (r >= 0 && (r & PT_INST_BIT)); }
 
 // 1/d of one axis for the slab test.  An axis the ray does not move along
 // (d = +-0, or |d| so small that 1/d overflows) gets +-1e20 with d's sign in
@@ -255,55 +238,78 @@ __device__ __forceinline__ bool ref_is_leaf(int32_t r) { return r < 0 && r != PT
 // entry beyond any tmax outside.
 __device__ __forceinline__ float slab_inv(float d) { return fabsf(d) > 1e-20f ? 1.f / d : copysignf(1e20f, d); }
 
-__device__ __forceinline__ void trav_init(TravRay &R, V3 o, V3 d, float tmin, float tmax, float time = 0.f) {
-  R.time = time;
-  R.o = o;
-  R.ow = o;
-  R.d = d;
-  R.dn = xnormalize(d);
-  R.inv = v3(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
-  R.oi = v3(-o.x * R.inv.x, -o.y * R.inv.y, -o.z * R.inv.z);
-  R.tmin = tmin;
-  R.tmax = tmax;
-  R.ref = 0;  // node 0 is the root (the host always emits at least one node)
-  R.sp = 0;
-  R.iters = 0;
-  R.found = false;
-  R.hit.t = FLT_MAX;
-  R.hit.prim = -1;
-  R.hit.u = R.hit.v = 0.f;
+// ------------------------------------------------- warp traversal of a queue
+// What a traversal warp keeps in shared memory.  A lane's ray is tested
+// against leaf items by whichever lane takes the leaf from the warp's list,
+// so everything the item tests read is here and not in the owner's registers.
+struct WarpRays {
+  float4 o[32];   // origin in the ray's current frame; w: time (motion blur)
+  float4 d[32];   // direction; w: tmin
+  float4 dn[32];  // normalised direction; w: tmax of any-hit rays
+  int32_t leaf[64];   // leaves reached and not yet tested, oldest first ...
+  uint8_t owner[64];  // ... and the lane whose ray reached each
+};
+// Closest-hit rays only: the nearest hit so far.
+struct WarpHits {
+  float4 hit[32];      // t, prim (int bits, -1: none), u, v
+  uint32_t tmax[32];   // float_key of the ray's tmax
+  int32_t who[32];     // tester whose hit the owner takes
+};
+enum TraceMode { TRACE_CLOSEST = 0, TRACE_ANY = 1, TRACE_MIXED = 2 };
+
+// Dynamic shared memory of a traversal block: the first PT_STACK_SHARED
+// entries of every thread's stack, the warps' records and, in scenes with
+// moving objects, the rays' world origins.
+inline size_t trace_smem(const SceneView &S, int threads, bool any_only = false) {
+  size_t per = PT_STACK_SHARED * sizeof(int32_t);
+  if (S.has_motion) per += 3 * sizeof(float);
+  return per * threads + (threads / 32) * (sizeof(WarpRays) + (any_only ? 0 : sizeof(WarpHits)));
 }
 
-__device__ __forceinline__ int32_t trav_pop(TravRay &R, const int32_t *stack, int stride) {
-  return R.sp == 0 ? PT_REF_EMPTY : stack[(--R.sp) * stride];
+// Unsigned key with the order of the floats (-0 as +0).
+__device__ __forceinline__ uint32_t float_key(float x) {
+  const uint32_t b = f2u(x + 0.f);
+  return b ^ ((uint32_t)((int32_t)b >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float key_float(uint32_t k) {
+  return u2f(k ^ ((k & 0x80000000u) ? 0x80000000u : 0xffffffffu));
 }
 
-// One node visit (or frame change).  R.ref must satisfy ref_is_node; after it
-// R.ref is the next reference (the nearest hit child for closest hit, the
-// first hit child in node order for any hit, else the top of the stack).
-// `stack` points at this thread's column of a shared array laid out
-// [PT_STACK][stride].  Returns false on a stack overflow (error flag set).
-template <bool ANY>
-__device__ __forceinline__ bool trav_node(const SceneView &S, TravRay &R, int32_t *stack, int stride, int *err) {
-  if (R.ref == PT_FRAME_END) {
-    // leaving a moving object's subtree: back to the world frame
-    R.o = R.ow;
-    R.oi = v3(-R.o.x * R.inv.x, -R.o.y * R.inv.y, -R.o.z * R.inv.z);
-    R.ref = trav_pop(R, stack, stride);
-    return true;
+__device__ __forceinline__ unsigned lanemask_lt() { return (1u << (threadIdx.x & 31)) - 1u; }
+
+// A lane's walk of the BVH4.
+struct TravRay {
+  V3 inv, oi;  // 1 / direction, -origin / direction in the current frame
+  float tmin, tmax;
+  int32_t ref;  // next reference: node (>= 0, PT_INST_BIT: entering a moving
+                // object), leaf (< 0), PT_FRAME_END or PT_REF_EMPTY
+  int sp;       // stack depth
+};
+
+// The per-thread stack: PT_STACK_SHARED entries in shared memory (column per
+// thread, conflict free) and the rest in local memory, which few rays reach
+// (leaves leave the stack as soon as they are met).
+struct TravStack {
+  int32_t *sh;  // this thread's column
+  int32_t deep[PT_STACK - PT_STACK_SHARED];
+  __device__ __forceinline__ void push(int &sp, int32_t r) {
+    if (sp < PT_STACK_SHARED) sh[sp * blockDim.x] = r;
+    else deep[sp - PT_STACK_SHARED] = r;
+    ++sp;
   }
-  if (R.ref & PT_INST_BIT) {
-    // entering a moving object's subtree: the ray in the object's frame at
-    // its time, until PT_FRAME_END comes off the stack
-    R.ref &= ~PT_INST_BIT;
-    if (R.sp + 1 > S.stack_entries) {
-      *err = 1;
-      return false;
-    }
-    stack[(R.sp++) * stride] = PT_FRAME_END;
-    R.o = moved_origin(S, (uint32_t)__ldg(S.node_motion + R.ref), R.ow, R.time);
-    R.oi = v3(-R.o.x * R.inv.x, -R.o.y * R.inv.y, -R.o.z * R.inv.z);
+  __device__ __forceinline__ int32_t pop(int &sp) {
+    if (sp == 0) return PT_REF_EMPTY;
+    --sp;
+    return sp < PT_STACK_SHARED ? sh[sp * blockDim.x] : deep[sp - PT_STACK_SHARED];
   }
+};
+
+// Visits node R.ref: afterwards R.ref is the next reference (SORTED: the
+// nearest hit child, the others pushed far first; else the first hit child in
+// node order), or the top of the stack when no child is hit.  Returns false
+// on a stack overflow.
+template <bool SORTED>
+__device__ __forceinline__ bool visit_node(const SceneView &S, TravRay &R, TravStack &K) {
   const float4 *np = reinterpret_cast<const float4 *>(S.nodes + R.ref);
   // The slab each child's entry and exit come from is fixed by the ray's
   // octant: with 1/d >= 0 along an axis the low plane is the near one
@@ -315,33 +321,31 @@ __device__ __forceinline__ bool trav_node(const SceneView &S, TravRay &R, int32_
   float4 nx = __ldg(np + sx), fx = __ldg(np + (sx ^ 1)), ny = __ldg(np + 2 + sy), fy = __ldg(np + 2 + (sy ^ 1));
   float4 nz = __ldg(np + 4 + sz), fz = __ldg(np + 4 + (sz ^ 1));
   // the children's traversal references, ready made by the upload (node
-  // index, leaf reference, or PT_REF_EMPTY for an empty slot)
+  // index or leaf reference; an empty slot's box is inverted and never hit)
   const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 7));
   const float nxa[4] = {nx.x, nx.y, nx.z, nx.w}, fxa[4] = {fx.x, fx.y, fx.z, fx.w};
   const float nya[4] = {ny.x, ny.y, ny.z, ny.w}, fya[4] = {fy.x, fy.y, fy.z, fy.w};
   const float nza[4] = {nz.x, nz.y, nz.z, nz.w}, fza[4] = {fz.x, fz.y, fz.z, fz.w};
-  const int rfa[4] = {rf.x, rf.y, rf.z, rf.w};
   const V3 inv = R.inv, oi = R.oi;
   const float tmin = R.tmin, tmax = R.tmax;
   // entry distance per child (+inf when missed or empty), kept in registers;
   // closest-hit visits near to far (sorting network), any-hit in node order.
   float d0, d1, d2, d3;
-  int32_t r0, r1, r2, r3;
-#define PT_CHILD(c, dd, rr)                                                                          \
+  int32_t r0 = rf.x, r1 = rf.y, r2 = rf.z, r3 = rf.w;
+#define PT_CHILD(c, dd)                                                                              \
   {                                                                                                  \
     float tn = fmaxf(fmaxf(fmaf(nxa[c], inv.x, oi.x), fmaf(nya[c], inv.y, oi.y)),                  \
                      fmaxf(fmaf(nza[c], inv.z, oi.z), tmin));                                        \
     float tf = fminf(fminf(fmaf(fxa[c], inv.x, oi.x), fmaf(fya[c], inv.y, oi.y)),                  \
                      fminf(fmaf(fza[c], inv.z, oi.z), tmax));                                        \
-    dd = (rfa[c] != PT_REF_EMPTY && tn <= tf) ? tn : INFINITY;                                      \
-    rr = rfa[c];                                                                                     \
+    dd = tn <= tf ? tn : INFINITY;                                                                   \
   }
-  PT_CHILD(0, d0, r0)
-  PT_CHILD(1, d1, r1)
-  PT_CHILD(2, d2, r2)
-  PT_CHILD(3, d3, r3)
+  PT_CHILD(0, d0)
+  PT_CHILD(1, d1)
+  PT_CHILD(2, d2)
+  PT_CHILD(3, d3)
 #undef PT_CHILD
-  if (!ANY) {
+  if (SORTED) {
 #define PT_CSWAP(da, ra, db, rb)   \
   if (db < da) {                   \
     float tt = da;                 \
@@ -358,91 +362,270 @@ __device__ __forceinline__ bool trav_node(const SceneView &S, TravRay &R, int32_
     PT_CSWAP(d1, r1, d2, r2)
 #undef PT_CSWAP
   }
-  const int nh = (d0 < INFINITY) + (d1 < INFINITY) + (d2 < INFINITY) + (d3 < INFINITY);
-  if (nh == 0) {
-    R.ref = trav_pop(R, stack, stride);
+  const bool h0 = d0 < INFINITY, h1 = d1 < INFINITY, h2 = d2 < INFINITY, h3 = d3 < INFINITY;
+  if (R.sp > PT_STACK_SHARED - 3) {
+    // near the end of the shared part: pushes that may go to local memory
+    if (R.sp > PT_STACK - 3) return false;
+    int32_t first = PT_REF_EMPTY;
+    bool have = false;
+    if (h3) { first = r3; have = true; }
+    if (h2) { if (have) K.push(R.sp, first); first = r2; have = true; }
+    if (h1) { if (have) K.push(R.sp, first); first = r1; have = true; }
+    if (h0) { if (have) K.push(R.sp, first); first = r0; have = true; }
+    R.ref = have ? first : K.pop(R.sp);
     return true;
   }
-  if (R.sp + nh - 1 > S.stack_entries) {
-    *err = 1;
-    return false;
-  }
-  // push the farther hits (far first), descend into the nearest
-  int32_t first = 0;
+  // push the other hits (far first, or in node order), descend into the first
   int sp = R.sp;
-  if (ANY) {
-    // node order: descend into the first hit child, push the others
-    bool have = false;
-    if (d3 < INFINITY) { first = r3; have = true; }
-    if (d2 < INFINITY) { if (have) stack[(sp++) * stride] = first; first = r2; have = true; }
-    if (d1 < INFINITY) { if (have) stack[(sp++) * stride] = first; first = r1; have = true; }
-    if (d0 < INFINITY) { if (have) stack[(sp++) * stride] = first; first = r0; have = true; }
+  int32_t *top = K.sh + sp * blockDim.x;
+  int32_t first = PT_REF_EMPTY;
+  if (SORTED) {
+    if (h3) { *top = r3; top += blockDim.x; ++sp; }
+    if (h2) { *top = r2; top += blockDim.x; ++sp; }
+    if (h1) { *top = r1; ++sp; }
+    first = r0;  // d0 is the smallest
+    R.sp = sp;
+    R.ref = h0 ? first : K.pop(R.sp);
   } else {
-    if (d3 < INFINITY) stack[(sp++) * stride] = r3;
-    if (d2 < INFINITY) stack[(sp++) * stride] = r2;
-    if (d1 < INFINITY) stack[(sp++) * stride] = r1;
-    first = r0;  // d0 is the smallest and finite (nh > 0)
+    bool have = false;
+    if (h3) { first = r3; have = true; }
+    if (h2) { if (have) { *top = first; top += blockDim.x; ++sp; } first = r2; have = true; }
+    if (h1) { if (have) { *top = first; top += blockDim.x; ++sp; } first = r1; have = true; }
+    if (h0) { if (have) { *top = first; ++sp; } first = r0; have = true; }
+    R.sp = sp;
+    R.ref = have ? first : K.pop(R.sp);
   }
-  R.sp = sp;
-  R.ref = first;
   return true;
 }
 
-// One traversal step of one ray: a node visit or the test of ONE item of the
-// current leaf (the leaf reference then advances to the leaf's next item, in
-// item order, so hits and their order are those of a whole-leaf test).  The
-// short step keeps a persistent warp's lanes close: a lane in a node and a
-// lane in a 4-item leaf cost one node visit + one item test per turn, not a
-// node visit + the leaf's whole loop.  Returns true
-// when the ray is finished: closest -> R.found / R.hit hold the nearest hit;
-// any -> R.found = occluded.  *err is set when the stack would overflow or
-// the iteration cap is reached (never expected); the ray is then finished
-// with what it has.
-template <bool ANY, bool CURVES = true>
-__device__ __forceinline__ bool trav_step(const SceneView &S, TravRay &R, int32_t *stack, int stride, int *err) {
-  if (++R.iters > S.trav_cap) {
-    *err = 2;
-    return true;
-  }
-  if (R.ref == PT_REF_EMPTY) return true;
-  if (ref_is_node(R.ref)) return !trav_node<ANY>(S, R, stack, stride, err);
-  // one leaf item per step, the leaf's items in order
-  const int32_t code = ~R.ref;  // first_item << 3 | count - 1
-  if (test_item<ANY, CURVES>(S, code >> 3, R.o, R.d, R.dn, R.tmin, R.tmax, R.hit, R.time)) {
-    R.found = true;
-    if (ANY) return true;
-  }
-  // the rest of the leaf, (first + 1, count - 1), is ~(code + 7) = ref - 7
-  R.ref = (code & 7) ? R.ref - 7 : trav_pop(R, stack, stride);
-  return false;
+// Lanes of a traversal warp that hold rays: all 32 while the queue has 32
+// rays or more for every warp of the grid, else an even share of the queue.
+__device__ __forceinline__ int warp_lanes(int n) {
+  const int warps = gridDim.x * (blockDim.x >> 5);
+  return min(32, max(1, (n + warps - 1) / warps));
 }
 
-// The kind of step a warp's lanes take this turn: leaf-item tests when at
-// least half of the active lanes stand at a leaf, else node visits (lanes
-// whose traversal has ended take theirs in node turns).  Every lane steps in
-// one code path per turn instead of the warp issuing both paths each turn for
-// its mix of lanes; lanes of the other kind wait a turn.  Each ray takes the
-// same steps in the same order either way, so hits are unchanged.  Called by
-// every lane of the warp.
-__device__ __forceinline__ bool warp_leaf_turn(bool active, int32_t ref) {
-  const unsigned am = __ballot_sync(0xffffffffu, active);
-  const unsigned lm = __ballot_sync(0xffffffffu, active && ref_is_leaf(ref));
-  return 2 * __popc(lm) >= __popc(am);
-}
-__device__ __forceinline__ bool lane_turn(bool active, int32_t ref, bool leaf_turn) {
-  return active && ref_is_leaf(ref) == leaf_turn;
-}
-
-// Whole traversal of one ray by one thread (batch test kernels).
-template <bool ANY>
-__device__ bool traverse(const SceneView &S, V3 o, V3 d, float tmin, float tmax, HitRec &hit,
-                         int32_t *stack, int stride, int *err, float time = 0.f) {
+// Traces a queue of n rays with persistent warps and dynamic ray fetch (Aila
+// and Laine, "Understanding the efficiency of ray traversal on GPUs", HPG
+// 2009, and the 2012 addendum): as soon as `refill` of 32 lanes are free, the
+// warp claims that many new rays with one atomic on *fetch.
+//
+// Node visits and item tests are separate phases of the warp.  A lane that
+// reaches a leaf appends it to the warp's list and goes on walking its other
+// nodes; once the list holds a leaf for every ray in flight (32 in a full
+// warp), or no lane has a node left to visit, the oldest 32 leaves are tested,
+// one per lane, whichever lane's ray they belong to.  So the item tests run
+// with a full warp and no lane waits at a leaf for the others.  A ray walks
+// its nodes with the tmax it had when the list was last tested, i.e. it
+// may visit nodes a tighter tmax would cull, whose items then fail; its leaves
+// are tested in the order it reached them, and of two equal-t hits the later
+// one wins, as in the reference's leaf loop.
+//
+// Measured against turns in which a warp either visits nodes or tests one item
+// per lane standing at a leaf (Cornell box, 256 x 256 x 64 spp): 15.3 -> 20.1
+// active threads per instruction in the shadow kernel, 8.29 -> 6.66 ms for
+// its 51 M rays (with the compact ray list, PT_FETCH_IDLE_SHADOW 16).  Rough
+// glass, 16.8 M paths: trace 16.5 -> 13.8 ms (39 M rays), shadow 16.8 ->
+// 13.3 ms (45 M).  Testing from 24 / 16 leaves on: shadow 13.0 / 13.1 ms on
+// the glass, 6.75 / 7.16 on Cornell, so 32 stays.  With 32 lanes always (no
+// even share) bounces of few rays wait for each other's leaves: the
+// 0.48 M-path glass frame 3.57 -> 3.9 ms.
+//
+// fetch_ray(r, o, d, tmin, tmax, time, any): loads ray r, false: no ray there.
+// done(found, hit): the lane's ray is finished.
+template <int MODE, bool CURVES, class Fetch, class Done>
+__device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch, int refill32, int *err, char *smem,
+                                           Fetch fetch_ray, Done done) {
+  const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  TravStack K;
+  K.sh = reinterpret_cast<int32_t *>(smem) + threadIdx.x;
+  smem += PT_STACK_SHARED * sizeof(int32_t) * blockDim.x;
+  WarpRays &W = reinterpret_cast<WarpRays *>(smem)[threadIdx.x >> 5];
+  smem += warps * sizeof(WarpRays);
+  WarpHits &H = reinterpret_cast<WarpHits *>(smem)[threadIdx.x >> 5];
+  if (MODE != TRACE_ANY) smem += warps * sizeof(WarpHits);
+  float *ow = reinterpret_cast<float *>(smem) + 3 * threadIdx.x;  // world origin (has_motion)
+  const int lanes = warp_lanes(n), refill = max(1, lanes * refill32 / 32);
   TravRay R;
-  trav_init(R, o, d, tmin, tmax, time);
-  while (!trav_step<ANY>(S, R, stack, stride, err)) {
+  R.ref = PT_REF_EMPTY;
+  R.sp = 0;
+  int iters = 0;
+  bool active = false;     // the lane has a ray in flight
+  bool pend = false;       // the list holds leaves of this lane's (last) ray
+  bool any = MODE == TRACE_ANY;
+  bool exhausted = false;  // the queue has no unclaimed rays
+  int qn = 0;              // leaves in the list
+  for (;;) {
+    // ---- rays that ended: nothing left to visit or to test
+    if (active && !pend && R.ref == PT_REF_EMPTY) {
+      HitRec h;
+      h.prim = -1;
+      if (MODE != TRACE_ANY) {
+        const float4 b = H.hit[lane];
+        h.t = b.x;
+        h.prim = __float_as_int(b.y);
+        h.u = b.z;
+        h.v = b.w;
+      }
+      done(h.prim >= 0, h);
+      active = false;
+    }
+    // ---- refill
+    const unsigned idle = __ballot_sync(0xffffffffu, !active && !pend);
+    const int in_flight = 32 - __popc(idle);
+    const int k = lanes - in_flight;  // rays to claim
+    if (!exhausted && k >= refill) {
+      int base = 0;
+      if (lane == 0) base = atomicAdd(fetch, k);
+      base = __shfl_sync(0xffffffffu, base, 0);
+      if (base + k >= n) exhausted = true;
+      const int rank = __popc(idle & lanemask_lt());
+      if (!active && !pend && rank < k) {
+        const int r = base + rank;
+        V3 o, d;
+        float time = 0.f;
+        if (r < n && fetch_ray(r, o, d, R.tmin, R.tmax, time, any)) {
+          const V3 dn = xnormalize(d);
+          W.o[lane] = make_float4(o.x, o.y, o.z, time);
+          W.d[lane] = make_float4(d.x, d.y, d.z, R.tmin);
+          W.dn[lane] = make_float4(dn.x, dn.y, dn.z, R.tmax);
+          if (MODE != TRACE_ANY) {
+            H.hit[lane] = make_float4(FLT_MAX, __int_as_float(-1), 0.f, 0.f);
+            H.tmax[lane] = float_key(R.tmax);
+            H.who[lane] = any ? -2 : -1;  // -2: an any-hit ray
+          }
+          if (S.has_motion) {
+            ow[0] = o.x;
+            ow[1] = o.y;
+            ow[2] = o.z;
+          }
+          R.inv = v3(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
+          R.oi = v3(-o.x * R.inv.x, -o.y * R.inv.y, -o.z * R.inv.z);
+          R.ref = 0;  // node 0 is the root (the host always emits at least one node)
+          R.sp = 0;
+          iters = 0;
+          active = true;
+        }
+      }
+      __syncwarp();
+      continue;
+    }
+    // ---- leaves reached go to the list
+    const bool leaf = active && ref_is_leaf(R.ref);
+    const unsigned lm = __ballot_sync(0xffffffffu, leaf);
+    if (leaf) {
+      const int at = qn + __popc(lm & lanemask_lt());
+      W.leaf[at] = R.ref;
+      W.owner[at] = (uint8_t)lane;
+      pend = true;
+      ++iters;
+      R.ref = K.pop(R.sp);
+    }
+    qn += __popc(lm);
+    // ---- a node visit for every lane that stands at one, or the item tests
+    const bool ready = active && ref_is_node(R.ref) && !(S.has_motion && pend && ref_is_frame(R.ref));
+    const unsigned rm = __ballot_sync(0xffffffffu, ready);
+    if (rm && qn < min(32, in_flight)) {
+      if (ready) {
+        bool ok = ++iters <= S.trav_cap;
+        if (!ok) *err = 2;
+        if (ok && S.has_motion && ref_is_frame(R.ref)) {
+          // the ray in the next frame: a moving object's at its time (until
+          // PT_FRAME_END comes off the stack), or back in the world's
+          V3 o = v3(ow[0], ow[1], ow[2]);
+          if (R.ref == PT_FRAME_END) {
+            R.ref = K.pop(R.sp);
+          } else {
+            R.ref &= ~PT_INST_BIT;
+            ok = R.sp < PT_STACK;
+            if (ok) K.push(R.sp, PT_FRAME_END);
+            o = moved_origin(S, (uint32_t)__ldg(S.node_motion + R.ref), o, W.o[lane].w);
+          }
+          R.oi = v3(-o.x * R.inv.x, -o.y * R.inv.y, -o.z * R.inv.z);
+          W.o[lane] = make_float4(o.x, o.y, o.z, W.o[lane].w);
+          if (!ok) *err = 1;
+        }
+        if (ok && ref_is_node(R.ref) && !(S.has_motion && ref_is_frame(R.ref))) {
+          ok = visit_node<MODE != TRACE_ANY>(S, R, K);
+          if (!ok) *err = 1;
+        }
+        if (!ok) {  // ended with what it has
+          R.ref = PT_REF_EMPTY;
+          R.sp = 0;
+        }
+      }
+      continue;
+    }
+    if (!qn) {
+      if (exhausted && idle == 0xffffffffu) break;
+      continue;
+    }
+    // ---- item tests: the oldest leaves, one per lane
+    __syncwarp();
+    const int m = min(qn, 32);
+    const int own = lane < m ? W.owner[lane] : 0;
+    const int32_t lref = lane < m ? W.leaf[lane] : 0;
+    const bool rest = 32 + lane < qn;
+    const int rown = rest ? W.owner[32 + lane] : 0;
+    const int32_t rleaf = rest ? W.leaf[32 + lane] : 0;
+    bool hit = false, eany = MODE == TRACE_ANY;
+    HitRec h;
+    if (lane < m) {
+      const float4 o4 = W.o[own], d4 = W.d[own];
+      float tm;
+      if (MODE == TRACE_MIXED) eany = H.who[own] == -2;
+      if (MODE == TRACE_ANY) tm = W.dn[own].w;
+      else tm = key_float(H.tmax[own]);
+      const V3 o = v3(o4.x, o4.y, o4.z), d = v3(d4.x, d4.y, d4.z);
+      const int32_t code = ~lref;  // first_item << 3 | count - 1
+      const int last = (code >> 3) + (code & 7);
+      for (int i = code >> 3; i <= last; ++i) {
+        if (test_item<CURVES>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w)) {
+          hit = true;
+          if (eany) break;
+          tm = h.t;
+        }
+      }
+    }
+    __syncwarp();
+    if (rest) {
+      W.owner[lane] = (uint8_t)rown;
+      W.leaf[lane] = rleaf;
+    }
+    qn -= m;
+    const unsigned left = __reduce_or_sync(0xffffffffu, rest ? 1u << rown : 0u);
+    if (MODE != TRACE_CLOSEST) {
+      const unsigned occ = __reduce_or_sync(0xffffffffu, hit && eany ? 1u << own : 0u);
+      if (active && any && (occ >> lane & 1u)) {
+        HitRec none;
+        none.prim = 0;
+        done(true, none);
+        active = false;
+        R.ref = PT_REF_EMPTY;
+        R.sp = 0;
+      }
+    }
+    if (MODE != TRACE_ANY) {
+      // the nearest of the leaves' hits per owner; of equal ones the latest
+      const bool cand = hit && !eany;
+      if (__any_sync(0xffffffffu, cand)) {
+        const uint32_t key = float_key(h.t);
+        if (cand) atomicMin(&H.tmax[own], key);
+        __syncwarp();
+        const bool best = cand && H.tmax[own] == key;
+        if (best) atomicMax(&H.who[own], lane);
+        __syncwarp();
+        if (best && H.who[own] == lane) H.hit[own] = make_float4(h.t, __int_as_float(h.prim), h.u, h.v);
+        __syncwarp();
+        if (active && !any) {
+          R.tmax = key_float(H.tmax[lane]);
+          H.who[lane] = -1;
+        }
+      }
+    }
+    pend = (left >> lane) & 1u;
+    __syncwarp();
   }
-  hit = R.hit;
-  return R.found;
 }
 
 }  // namespace pt
