@@ -381,7 +381,8 @@ int pt_load_image(const char *path, int32_t flip_y, int32_t is_hdr, float **texe
                   int32_t *height);
 int pt_free_image(float *texels);
 /* Counts of the flattened scene: [0] triangles, [1] quads, [2] spheres,
- * [3] BVH4 nodes, [4] lights, [5] device bytes. */
+ * [3] BVH4 nodes, [4] lights, [5] bytes of the flattened scene (its BVH4 nodes
+ * counted at 128 bytes as built; the device keeps them packed to 64). */
 int pt_scene_info(void *ctx, int32_t scene_id, int64_t *out6);
 
 /* Renders one job synchronously (replaces the pixel loop of

@@ -1504,17 +1504,24 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
 
   // upload
   auto up = [&](const auto &v) { return device ? dupload(v, S->owned, st) : nullptr; };
-  {
-    // the device copy carries each child's traversal reference in place of
-    // its count (the node visit then needs neither the child row nor any
-    // decoding); the host tree and its hash keep (child, count)
-    std::vector<Bvh4Node> dev = out.nodes;
-    for (Bvh4Node &N : dev)
-      for (int k = 0; k < 4; ++k) {
-        if (N.count[k] > 8) fail(PT_ERR_INVALID, "leaf of more than 8 items");
-        N.count[k] = trav_ref(N.child[k], N.count[k]);
-      }
-    S->nodes = up(dev);
+  for (const Bvh4Node &N : out.nodes)
+    for (int k = 0; k < 4; ++k)
+      if (N.count[k] > 8) fail(PT_ERR_INVALID, "leaf of more than 8 items");
+  std::vector<void *> staged;  // freed when the scene is up
+  struct Freed {
+    std::vector<void *> &v;
+    ~Freed() {
+      for (void *p : v) cudaFree(p);
+    }
+  } freed{staged};
+  if (device) {
+    // packed on the device; the host tree and its hash keep the float boxes
+    const Bvh4Node *wide = dupload(out.nodes, staged, st);
+    void *packed = nullptr;
+    cuda_check(cudaMalloc(&packed, sizeof(PackedNode) * out.nodes.size()), "cudaMalloc(nodes)");
+    S->owned.push_back(packed);
+    S->nodes = static_cast<PackedNode *>(packed);
+    launch_pack_nodes(wide, (int)out.nodes.size(), S->nodes, st);
   }
   S->items = up(items);
   S->shade = up(shade);

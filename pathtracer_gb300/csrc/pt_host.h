@@ -38,7 +38,7 @@ void validate_job(const pt_job_desc &j);
 // A flattened scene resident in HBM.
 struct Scene {
   SceneView view;
-  Bvh4Node *nodes = nullptr;
+  PackedNode *nodes = nullptr;
   Item *items = nullptr;
   PrimShade *shade = nullptr;
   MatRec *materials = nullptr;

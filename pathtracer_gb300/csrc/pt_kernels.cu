@@ -70,13 +70,13 @@ void launch_path_samples(const DeviceJob &J, long long first, int n, int dims, i
 
 // The batch ray queries: closest hits or occlusion of n given rays, *fetch = 0
 // at the start.
-template <bool ANY>
+template <bool ANY, bool CURVES, bool MOTION>
 __global__ void __launch_bounds__(128) k_trace_test(SceneView S, const float *rays, const float *tmaxs, int n,
                                                     float tmin, float tmax, float *t_out, int *prim_out, float *uv_out,
                                                     uint8_t *occ, int *fetch, int *err) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
   int i = 0;
-  trace_rays<ANY ? TRACE_ANY : TRACE_CLOSEST, true>(
+  trace_rays<ANY ? TRACE_ANY : TRACE_CLOSEST, CURVES, MOTION>(
       S, n, fetch, ANY ? PT_FETCH_IDLE_SHADOW : PT_FETCH_IDLE, err, smem,
       [&](int r, V3 &o, V3 &d, float &t0, float &t1, float &, bool &) {
         i = r;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(128) k_intersect(SceneView S, const float *ray
                                                    uint8_t *front, int *fetch, int *err) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
   int i = 0;
-  trace_rays<TRACE_CLOSEST, true>(
+  trace_rays<TRACE_CLOSEST, true, true>(
       S, n, fetch, PT_FETCH_IDLE, err, smem,
       [&](int r, V3 &o, V3 &d, float &t0, float &t1, float &, bool &) {
         i = r;
@@ -140,7 +140,7 @@ __global__ void __launch_bounds__(128) k_intersect(SceneView S, const float *ray
 void launch_intersect(const SceneView &S, const float *rays, int n, float tmin, float tmax, float *t, int *prim,
                       float *pos, float *nrm, uint8_t *front, int *fetch, int *err, cudaStream_t st) {
   cudaMemsetAsync(fetch, 0, sizeof(int), st);
-  k_intersect<<<grid_for(n, 128, 152 * 7), 128, trace_smem(S, 128), st>>>(S, rays, n, tmin, tmax, t, prim, pos, nrm,
+  k_intersect<<<grid_for(n, 128, 152 * 7), 128, trace_smem(128), st>>>(S, rays, n, tmin, tmax, t, prim, pos, nrm,
                                                                          front, fetch, err);
 }
 
@@ -282,10 +282,10 @@ __global__ void k_sort_scatter(Queues Q, int qsel) {
 
 // k_trace_shadow, k_shadow_resolve, k_film: their bodies are in pt_wave.cuh
 // (trace_shadow_body, shadow_resolve_body, film_body).
-template <bool CURVES>
-__global__ void __launch_bounds__(128) k_trace_shadow(SceneView S, Queues Q) {
+template <bool CURVES, bool MOTION>
+__global__ void __launch_bounds__(128, CURVES ? 7 : 8) k_trace_shadow(SceneView S, Queues Q) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
-  trace_shadow_body<CURVES>(S, Q, smem);
+  trace_shadow_body<CURVES, MOTION>(S, Q, smem);
 }
 __global__ void k_shadow_resolve(Queues Q, int LN) { shadow_resolve_body(Q, LN); }
 __global__ void k_film(DeviceJob J, Queues Q, long long g0, int n, long long slot0, float *film) {
@@ -366,7 +366,16 @@ __global__ void k_tonemap(const float *film, int W, int H, float inv_gamma, uint
   }
 }
 
+// The traversal's nodes from the built ones, one per thread (a scene upload).
+__global__ void k_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = pack_node(nodes[i]);
+}
+
 // ---------------------------------------------------------------- launchers
+void launch_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out, cudaStream_t st) {
+  k_pack_nodes<<<grid_for(n, 128, 152 * 16), 128, 0, st>>>(nodes, n, out);
+}
+
 void upload_halton_tables(const HaltonTables &T, cudaStream_t st) {
   cudaMemcpyToSymbolAsync(c_halton, &T, sizeof(T), 0, cudaMemcpyHostToDevice, st);
 }
@@ -384,11 +393,21 @@ void launch_trace_test(const SceneView &S, bool any, const float *rays, const fl
                        cudaStream_t st) {
   const int g = grid_for(n, 128, 152 * 7);
   cudaMemsetAsync(fetch, 0, sizeof(int), st);
-  if (any)
-    k_trace_test<true><<<g, 128, trace_smem(S, 128, true), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, fetch,
-                                                                 err);
-  else
-    k_trace_test<false><<<g, 128, trace_smem(S, 128), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, fetch, err);
+#define PT_RUN(C, M)                                                                                             \
+  if (any)                                                                                                       \
+    k_trace_test<true, C, M><<<g, 128, trace_smem(128, true), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, \
+                                                                       occ, fetch, err);                         \
+  else                                                                                                           \
+    k_trace_test<false, C, M><<<g, 128, trace_smem(128), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, \
+                                                                  fetch, err)
+  if (S.curves) {
+    PT_RUN(true, true);
+  } else if (S.has_motion) {
+    PT_RUN(false, true);
+  } else {
+    PT_RUN(false, false);
+  }
+#undef PT_RUN
 }
 
 void launch_bsdf_eval(const MatRec *m, int n, const float *wo, const float *wi, const float *nrm,
@@ -427,10 +446,9 @@ void launch_sort(const SceneView &S, const Queues &Q, int qsel, const LaunchCfg 
 }
 
 void launch_shadow(const SceneView &S, const Queues &Q, int LN, const LaunchCfg &cfg, cudaStream_t st) {
-  if (S.curves)
-    k_trace_shadow<true><<<cfg.trace_blocks, 128, trace_smem(S, 128, true), st>>>(S, Q);
-  else
-    k_trace_shadow<false><<<cfg.trace_blocks, 128, trace_smem(S, 128, true), st>>>(S, Q);
+#define PT_RUN(C, M) k_trace_shadow<C, M><<<cfg.trace_blocks, 128, trace_smem(128, true), st>>>(S, Q)
+  PT_BY_SCENE(S, PT_RUN);
+#undef PT_RUN
   k_shadow_resolve<<<cfg.max_blocks_simple, 256, 0, st>>>(Q, LN);
 }
 void launch_shadow_resolve(const Queues &Q, int LN, const LaunchCfg &cfg, cudaStream_t st) {
@@ -463,19 +481,17 @@ void launch_tonemap(const float *film, int W, int H, float gamma, uint8_t *out, 
 
 void kernel_attributes(KernelInfo *info) {
   cudaFuncAttributes a;
-  cudaFuncGetAttributes(&a, k_trace_closest<false, false>);
+  cudaFuncGetAttributes(&a, k_trace_closest<false, false, false>);
   info->trace_regs = a.numRegs;
   cudaFuncGetAttributes(&a, k_shade<-1, false>);
   info->shade_regs = a.numRegs;
   int nb = 0;
-  SceneView any_scene{};  // occupancy at the largest shared memory (the grids must fit every scene)
-  any_scene.has_motion = 1;
-  const size_t smax = trace_smem(any_scene, 128);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_closest<false, false>, 128, smax);
+  const size_t smax = trace_smem(128);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_closest<false, false, false>, 128, smax);
   info->trace_blocks_per_sm = nb;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade<-1, false>, 128, 0);
   info->shade_blocks_per_sm = nb;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_shadow<false>, 128, smax);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_shadow<false, false>, 128, smax);
   info->shadow_blocks_per_sm = nb;
   int *fb = info->shade_fam_blocks_per_sm;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[0], k_shade<0, false>, 128, 0);

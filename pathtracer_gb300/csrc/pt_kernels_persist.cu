@@ -87,27 +87,27 @@ struct NoReset {
 // The stages as separately compiled functions: each gets its own register
 // allocation (the traversal does not inherit the shading's register pressure
 // and spills), and reads the kernel's parameters in place (__grid_constant__).
-template <bool CURVES>
+template <bool CURVES, bool MOTION>
 __device__ __noinline__ void st_trace(const SceneView &S, const DeviceJob &none, const JobTable &T, const Queues &Q,
                                       int qsel, int b, long long g0, char *smem) {
   if (b > 0)
-    trace_pair_body<true, CURVES>(S, none, T, Q, qsel, b, g0, smem);
+    trace_pair_body<true, CURVES, MOTION>(S, none, T, Q, qsel, b, g0, smem);
   else
-    trace_closest_body<true, CURVES>(S, none, T, Q, qsel, b, g0, smem);
+    trace_closest_body<true, CURVES, MOTION>(S, none, T, Q, qsel, b, g0, smem);
 }
 __device__ __noinline__ void st_shade(const SceneView &S, const DeviceJob &none, const JobTable &T, const Queues &Q,
                                       int qsel, int b, long long g0) {
   shade_body<-1, true>(S, none, T, Q, qsel, b, g0);
 }
-template <bool CURVES>
+template <bool CURVES, bool MOTION>
 __device__ __noinline__ void st_shadow(const SceneView &S, const Queues &Q, char *smem) {
-  trace_shadow_body<CURVES>(S, Q, smem);
+  trace_shadow_body<CURVES, MOTION>(S, Q, smem);
 }
 
 // The whole group: for each wave of `wave` paths over [0, total), camera ->
 // per bounce (trace [+ previous shadow rays] -> resolve -> shade) -> last
 // shadow rays -> resolve -> films.
-template <bool CURVES>
+template <bool CURVES, bool MOTION>
 __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
     k_group_persistent(const __grid_constant__ SceneView S, const __grid_constant__ JobTable T,
                        const __grid_constant__ Queues Q, float *const *films, long long total, int wave, int LN,
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
     if (!grid_sync(bar, [=] { cnt[1] = 0; cnt[2] = 0; cnt[3] = 0; cnt[4] = 0; cnt[5] = 0; })) return;
     int qsel = 0;
     for (int b = 0; b < bounces; ++b) {
-      st_trace<CURVES>(S, none, T, Q, qsel, b, g0, smem);
+      st_trace<CURVES, MOTION>(S, none, T, Q, qsel, b, g0, smem);
       const int nq = qsel ^ 1;
       if (!grid_sync(bar, [=] { cnt[nq] = 0; cnt[4] = 0; })) return;
       if (b > 0) {
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
       if (!grid_sync(bar, NoReset())) return;
       qsel = nq;
     }
-    st_shadow<CURVES>(S, Q, smem);
+    st_shadow<CURVES, MOTION>(S, Q, smem);
     if (!grid_sync(bar, NoReset())) return;
     shadow_resolve_body(Q, LN);
     if (!grid_sync(bar, NoReset())) return;
@@ -151,11 +151,11 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
 
 int persistent_grid(const SceneView &S, int num_sms) {
   int per = 0;
-  const size_t smem = trace_smem(S, PT_PERSIST_THREADS);
+  const size_t smem = trace_smem(PT_PERSIST_THREADS);
   if (S.curves)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_group_persistent<true>, PT_PERSIST_THREADS, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_group_persistent<true, true>, PT_PERSIST_THREADS, smem);
   else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_group_persistent<false>, PT_PERSIST_THREADS, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_group_persistent<false, true>, PT_PERSIST_THREADS, smem);
   return std::max(1, per) * num_sms;
 }
 
@@ -168,9 +168,9 @@ cudaError_t launch_group_persistent(const SceneView &S, const JobTable &T, const
   float *const *f = d_films;
   GridBarrier *b = static_cast<GridBarrier *>(d_barrier);
   void *args[] = {&s, &t, &q, &f, &total, &wave, &LN, &bounces, &b};
-  const void *fn = S.curves ? (const void *)k_group_persistent<true> : (const void *)k_group_persistent<false>;
+  const void *fn = S.curves ? (const void *)k_group_persistent<true, true> : (const void *)k_group_persistent<false, true>;
   return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PT_PERSIST_THREADS), args,
-                                     trace_smem(S, PT_PERSIST_THREADS), st);
+                                     trace_smem(PT_PERSIST_THREADS), st);
 }
 
 }  // namespace pt

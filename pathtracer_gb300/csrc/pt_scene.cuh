@@ -1,8 +1,8 @@
 // pt_scene.cuh -- device layout of a flattened scene and of a render job.
 //
 // A scene is uploaded once (pt_scene_upload) and stays resident in HBM:
-//   * BVH4 nodes, 128 B each (one L2 line): child boxes as SoA float4 rows,
-//     child references and leaf item counts;
+//   * BVH4 nodes, 64 B each (PackedNode, pt_node.cuh): child boxes as bytes on
+//     the node's grid and child references;
 //   * leaf items, 48 B each (3 x float4), in leaf order: a triangle keeps
 //     v0, e1 = v1 - v0, e2 = v2 - v0 exactly as the reference's hitTriangle
 //     computes them (meshBVH.cpp:91-93), an AARectangle its plane and
@@ -12,6 +12,7 @@
 //     lightDiscovery.hpp:5-81) and the environment map with its alias table.
 #pragma once
 #include "pt_common.cuh"
+#include "pt_node.cuh"
 
 // Largest traversal stack, in entries per thread: a BVH4 of depth D needs at
 // most 3 * D + 1; scene upload rejects deeper trees.  The first
@@ -24,28 +25,6 @@
 namespace pt {
 
 enum ItemType : int32_t { ITEM_TRI = 0, ITEM_QUAD = 1, ITEM_SPHERE = 2, ITEM_CURVE = 3 };
-
-struct alignas(128) Bvh4Node {
-  float lo_x[4], hi_x[4];
-  float lo_y[4], hi_y[4];
-  float lo_z[4], hi_z[4];
-  int32_t child[4];  // internal: node index; leaf: first item index
-  int32_t count[4];  // internal: 0; leaf: number of items; empty slot: -1 --
-                     // in the uploaded copy: each child's traversal reference
-                     // (trav_ref), which the node visit reads as is
-};
-static_assert(sizeof(Bvh4Node) == 128, "BVH4 node must be one 128-byte line");
-
-// Traversal references (a node's children on the device, the stack): a node
-// index (>= 0; PT_INST_BIT: entering a moving object), a leaf
-// ~(first_item << 3 | count - 1) (count <= 8), PT_FRAME_END (stack only) or
-// PT_REF_EMPTY (an empty child slot; as the next reference: nothing pending).
-#define PT_REF_EMPTY ((int32_t)0x80000001)
-PT_HD int32_t leaf_ref(int32_t first, int32_t count) { return ~((first << 3) | (count - 1)); }
-// A child's reference from its (child, count) pair.
-PT_HD int32_t trav_ref(int32_t child, int32_t count) {
-  return count < 0 ? PT_REF_EMPTY : count == 0 ? child : leaf_ref(child, count);
-}
 
 // Leaf item (48 B).  a.w / b.w carry the primitive id and the item type as
 // integer bits.
@@ -131,7 +110,7 @@ struct alignas(16) TexRec {
 enum UvKind : int32_t { PT_UV_TRI = 1, PT_UV_PLANAR = 2, PT_UV_QUAD = 3, PT_UV_SPHERE = 4 };
 
 struct SceneView {
-  const Bvh4Node *nodes;
+  const PackedNode *nodes;
   const Item *items;
   const PrimShade *shade;
   const MatRec *materials;

@@ -194,13 +194,14 @@ __device__ __forceinline__ V3 moved_origin(const SceneView &S, uint32_t motion, 
 // Tests leaf item `idx` against a ray (origin o in its current frame); a
 // hit in [tmin, tmax] fills `hit`.  dn points at the ray's normalised
 // direction (rectangles and spheres read it).  CURVES = false compiles the
-// curve test out (curve items then never hit).
-template <bool CURVES>
+// curve test out (curve items then never hit), MOTION = false the moving
+// primitives.
+template <bool CURVES, bool MOTION>
 __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V3 d, const float4 *dn4, float tmin,
                                           float tmax, HitRec &hit, float time) {
   Item it = load_item(S.items, idx);
   const int type = (int)f2u(it.b[3]);
-  const uint32_t motion = f2u(it.c[3]);
+  const uint32_t motion = MOTION ? f2u(it.c[3]) : 0u;
   const V3 o = motion ? moved_origin(S, motion, o_w, time) : o_w;
   float t, u = 0.f, v = 0.f;
   bool h;
@@ -255,14 +256,22 @@ struct WarpHits {
   uint32_t tmax[32];   // float_key of the ray's tmax
   int32_t who[32];     // tester whose hit the owner takes
 };
+// Lanes (of 32) below which a walk pauses to see whether others have ended.
+#define PT_WALK_MIN 12
+// One kernel per kind of scene: PT_BY_SCENE(S, RUN) expands RUN(CURVES, MOTION).
+#define PT_BY_SCENE(S, RUN)          \
+  do {                               \
+    if ((S).curves) RUN(true, true); \
+    else if ((S).has_motion) RUN(false, true); \
+    else RUN(false, false);          \
+  } while (0)
 enum TraceMode { TRACE_CLOSEST = 0, TRACE_ANY = 1, TRACE_MIXED = 2 };
 
 // Dynamic shared memory of a traversal block: the first PT_STACK_SHARED
-// entries of every thread's stack, the warps' records and, in scenes with
-// moving objects, the rays' world origins.
-inline size_t trace_smem(const SceneView &S, int threads, bool any_only = false) {
-  size_t per = PT_STACK_SHARED * sizeof(int32_t);
-  if (S.has_motion) per += 3 * sizeof(float);
+// entries of every thread's stack, the warps' records and the rays' world
+// origins (kernels for moving objects).
+inline size_t trace_smem(int threads, bool any_only = false) {
+  const size_t per = PT_STACK_SHARED * sizeof(int32_t) + 3 * sizeof(float);
   return per * threads + (threads / 32) * (sizeof(WarpRays) + (any_only ? 0 : sizeof(WarpHits)));
 }
 
@@ -304,47 +313,76 @@ struct TravStack {
   }
 };
 
+// Two floats in a register pair.
+__device__ __forceinline__ uint64_t pack2(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+// (u0, u1) * a + c, one instruction for the pair (both rounded as fmaf): a
+// node visit's 24 plane distances take 12 issue slots.  The traversal issues
+// in 72-84 % of its cycles; rough glass trace 11.9 -> 11.4 ms, shadow 10.6 ->
+// 10.2, Cornell 7.19 -> 6.90.
+__device__ __forceinline__ void fma2(uint32_t u0, uint32_t u1, uint64_t a, uint64_t c, float &t0, float &t1) {
+  asm("{ .reg .b64 u, t;\n mov.b64 u, {%2, %3};\n fma.rn.f32x2 t, u, %4, %5;\n mov.b64 {%0, %1}, t; }"
+      : "=f"(t0), "=f"(t1)
+      : "r"(u0), "r"(u1), "l"(a), "l"(c));
+}
+// 32 bytes of a node with one load.
+__device__ __forceinline__ void ld32b(const void *p, uint32_t *v) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "l"(p));
+}
+
 // Visits node R.ref: afterwards R.ref is the next reference (SORTED: the
 // nearest hit child, the others pushed far first; else the first hit child in
 // node order), or the top of the stack when no child is hit.  Returns false
 // on a stack overflow.
 template <bool SORTED>
 __device__ __forceinline__ bool visit_node(const SceneView &S, TravRay &R, TravStack &K) {
-  const float4 *np = reinterpret_cast<const float4 *>(S.nodes + R.ref);
-  // The slab each child's entry and exit come from is fixed by the ray's
-  // octant: with 1/d >= 0 along an axis the low plane is the near one
-  // (fma is monotonic, so fmaf(lo, inv, oi) <= fmaf(hi, inv, oi) and the
-  // min / max the general slab test takes per child equal these picks), so
-  // the near and far rows are loaded by the sign of 1/d and no per-child
-  // min / max is spent choosing them (measured: traversal stage -5.5 %).
-  const int sx = signbit(R.inv.x) ? 1 : 0, sy = signbit(R.inv.y) ? 1 : 0, sz = signbit(R.inv.z) ? 1 : 0;
-  float4 nx = __ldg(np + sx), fx = __ldg(np + (sx ^ 1)), ny = __ldg(np + 2 + sy), fy = __ldg(np + 2 + (sy ^ 1));
-  float4 nz = __ldg(np + 4 + sz), fz = __ldg(np + 4 + (sz ^ 1));
-  // the children's traversal references, ready made by the upload (node
-  // index or leaf reference; an empty slot's box is inverted and never hit)
-  const int4 rf = __ldg(reinterpret_cast<const int4 *>(np + 7));
-  const float nxa[4] = {nx.x, nx.y, nx.z, nx.w}, fxa[4] = {fx.x, fx.y, fx.z, fx.w};
-  const float nya[4] = {ny.x, ny.y, ny.z, ny.w}, fya[4] = {fy.x, fy.y, fy.z, fy.w};
-  const float nza[4] = {nz.x, nz.y, nz.z, nz.w}, fza[4] = {fz.x, fz.y, fz.z, fz.w};
-  const V3 inv = R.inv, oi = R.oi;
+  uint32_t w[16];
+  ld32b(S.nodes + R.ref, w);
+  ld32b(reinterpret_cast<const char *>(S.nodes + R.ref) + 32, w + 8);
+  // Per axis, plane q at the ray parameter fma(1 + q 2^-15, a, c); the slab a
+  // child's entry and exit come from is fixed by the ray's octant (with 1/d >= 0
+  // the low plane is the near one; fma is monotonic, so these are the values
+  // a min / max of both planes would pick).
+  const V3 a = v3(u2f(w[3]) * R.inv.x, u2f(w[4]) * R.inv.y, u2f(w[5]) * R.inv.z);
+  const V3 c = v3(fmaf(u2f(w[0]), R.inv.x, R.oi.x), fmaf(u2f(w[1]), R.inv.y, R.oi.y),
+                  fmaf(u2f(w[2]), R.inv.z, R.oi.z));
+  const bool sx = signbit(R.inv.x), sy = signbit(R.inv.y), sz = signbit(R.inv.z);
+  const uint32_t nx = sx ? w[7] : w[6], fx = sx ? w[6] : w[7];
+  const uint32_t ny = sy ? w[9] : w[8], fy = sy ? w[8] : w[9];
+  const uint32_t nz = sz ? w[11] : w[10], fz = sz ? w[10] : w[11];
   const float tmin = R.tmin, tmax = R.tmax;
   // entry distance per child (+inf when missed or empty), kept in registers;
   // closest-hit visits near to far (sorting network), any-hit in node order.
   float d0, d1, d2, d3;
-  int32_t r0 = rf.x, r1 = rf.y, r2 = rf.z, r3 = rf.w;
-#define PT_CHILD(c, dd)                                                                              \
+  int32_t r0 = (int32_t)w[12], r1 = (int32_t)w[13], r2 = (int32_t)w[14], r3 = (int32_t)w[15];
+#define PT_PLANE(q, k) __byte_perm(q, 0x3f800000u, 0x7604 | (k << 4))
+  const uint64_t ax2 = pack2(a.x, a.x), ay2 = pack2(a.y, a.y), az2 = pack2(a.z, a.z);
+  const uint64_t cx2 = pack2(c.x, c.x), cy2 = pack2(c.y, c.y), cz2 = pack2(c.z, c.z);
+#define PT_PAIR(q, k, a2, c2, t0, t1) fma2(PT_PLANE(q, k), PT_PLANE(q, k + 1), a2, c2, t0, t1)
+#define PT_CHILDREN(k, da, db)                                                                       \
   {                                                                                                  \
-    float tn = fmaxf(fmaxf(fmaf(nxa[c], inv.x, oi.x), fmaf(nya[c], inv.y, oi.y)),                  \
-                     fmaxf(fmaf(nza[c], inv.z, oi.z), tmin));                                        \
-    float tf = fminf(fminf(fmaf(fxa[c], inv.x, oi.x), fmaf(fya[c], inv.y, oi.y)),                  \
-                     fminf(fmaf(fza[c], inv.z, oi.z), tmax));                                        \
-    dd = tn <= tf ? tn : INFINITY;                                                                   \
+    float ex, ey, ez, gx, gy, gz, px, py, pz, qx, qy, qz;                                            \
+    PT_PAIR(nx, k, ax2, cx2, ex, gx);                                                                \
+    PT_PAIR(ny, k, ay2, cy2, ey, gy);                                                                \
+    PT_PAIR(nz, k, az2, cz2, ez, gz);                                                                \
+    PT_PAIR(fx, k, ax2, cx2, px, qx);                                                                \
+    PT_PAIR(fy, k, ay2, cy2, py, qy);                                                                \
+    PT_PAIR(fz, k, az2, cz2, pz, qz);                                                                \
+    const float na = fmaxf(fmaxf(ex, ey), fmaxf(ez, tmin)), fa = fminf(fminf(px, py), fminf(pz, tmax)); \
+    const float nb = fmaxf(fmaxf(gx, gy), fmaxf(gz, tmin)), fb = fminf(fminf(qx, qy), fminf(qz, tmax)); \
+    da = na <= fa ? na : INFINITY;                                                                   \
+    db = nb <= fb ? nb : INFINITY;                                                                   \
   }
-  PT_CHILD(0, d0)
-  PT_CHILD(1, d1)
-  PT_CHILD(2, d2)
-  PT_CHILD(3, d3)
-#undef PT_CHILD
+  PT_CHILDREN(0, d0, d1)
+  PT_CHILDREN(2, d2, d3)
+#undef PT_CHILDREN
+#undef PT_PAIR
+#undef PT_PLANE
   if (SORTED) {
 #define PT_CSWAP(da, ra, db, rb)   \
   if (db < da) {                   \
@@ -431,9 +469,16 @@ __device__ __forceinline__ int warp_lanes(int n) {
 // even share) bounces of few rays wait for each other's leaves: the
 // 0.48 M-path glass frame 3.57 -> 3.9 ms.
 //
+// A turn of the walk does one node visit; done rays and the refill are looked at
+// only when PT_WALK_MIN lanes or fewer still walk (rough glass trace 12.9 ->
+// 12.2 ms, shadow 11.5 -> 10.6 against a look every turn; 8 / 16 / 20 lanes are
+// within 1 % but for closest hits at 20, +3 %).  MOTION = false (scenes without
+// moving objects) compiles the changes of frame out: trace 11.4 -> 10.9 ms, the
+// 0.48 M-path glass frame's 1.60 -> 1.49.
+//
 // fetch_ray(r, o, d, tmin, tmax, time, any): loads ray r, false: no ray there.
 // done(found, hit): the lane's ray is finished.
-template <int MODE, bool CURVES, class Fetch, class Done>
+template <int MODE, bool CURVES, bool MOTION, class Fetch, class Done>
 __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch, int refill32, int *err, char *smem,
                                            Fetch fetch_ray, Done done) {
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -444,8 +489,9 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
   smem += warps * sizeof(WarpRays);
   WarpHits &H = reinterpret_cast<WarpHits *>(smem)[threadIdx.x >> 5];
   if (MODE != TRACE_ANY) smem += warps * sizeof(WarpHits);
-  float *ow = reinterpret_cast<float *>(smem) + 3 * threadIdx.x;  // world origin (has_motion)
+  float *ow = reinterpret_cast<float *>(smem) + 3 * threadIdx.x;  // world origin (MOTION)
   const int lanes = warp_lanes(n), refill = max(1, lanes * refill32 / 32);
+  const int walk_min = lanes * PT_WALK_MIN / 32;
   TravRay R;
   R.ref = PT_REF_EMPTY;
   R.sp = 0;
@@ -457,6 +503,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
   int qn = 0;              // leaves in the list
   for (;;) {
     // ---- rays that ended: nothing left to visit or to test
+    if (active && !pend && R.ref == PT_REF_EMPTY && R.sp > 0) R.ref = K.pop(R.sp);
     if (active && !pend && R.ref == PT_REF_EMPTY) {
       HitRec h;
       h.prim = -1;
@@ -494,7 +541,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
             H.tmax[lane] = float_key(R.tmax);
             H.who[lane] = any ? -2 : -1;  // -2: an any-hit ray
           }
-          if (S.has_motion) {
+          if (MOTION) {
             ow[0] = o.x;
             ow[1] = o.y;
             ow[2] = o.z;
@@ -510,26 +557,30 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
       __syncwarp();
       continue;
     }
-    // ---- leaves reached go to the list
-    const bool leaf = active && ref_is_leaf(R.ref);
-    const unsigned lm = __ballot_sync(0xffffffffu, leaf);
-    if (leaf) {
-      const int at = qn + __popc(lm & lanemask_lt());
-      W.leaf[at] = R.ref;
-      W.owner[at] = (uint8_t)lane;
-      pend = true;
-      ++iters;
-      R.ref = K.pop(R.sp);
-    }
-    qn += __popc(lm);
-    // ---- a node visit for every lane that stands at one, or the item tests
-    const bool ready = active && ref_is_node(R.ref) && !(S.has_motion && pend && ref_is_frame(R.ref));
-    const unsigned rm = __ballot_sync(0xffffffffu, ready);
-    if (rm && qn < min(32, in_flight)) {
+    // ---- walk: leaves reached go to the list, a node visit for every lane
+    // that stands at one; until the list is full, or so few lanes walk on that
+    // others may have ended
+    const int full = min(32, in_flight);
+    unsigned rm;
+    for (;;) {
+      const bool leaf = active && ref_is_leaf(R.ref);
+      const unsigned lm = __ballot_sync(0xffffffffu, leaf);
+      if (leaf) {
+        const int at = qn + __popc(lm & lanemask_lt());
+        W.leaf[at] = R.ref;
+        W.owner[at] = (uint8_t)lane;
+        pend = true;
+        ++iters;
+        R.ref = K.pop(R.sp);
+      }
+      qn += __popc(lm);
+      const bool ready = active && ref_is_node(R.ref) && !(MOTION && pend && ref_is_frame(R.ref));
+      rm = __ballot_sync(0xffffffffu, ready);
+      if (!rm || qn >= full) break;
       if (ready) {
         bool ok = ++iters <= S.trav_cap;
         if (!ok) *err = 2;
-        if (ok && S.has_motion && ref_is_frame(R.ref)) {
+        if (ok && MOTION && ref_is_frame(R.ref)) {
           // the ray in the next frame: a moving object's at its time (until
           // PT_FRAME_END comes off the stack), or back in the world's
           V3 o = v3(ow[0], ow[1], ow[2]);
@@ -545,7 +596,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           W.o[lane] = make_float4(o.x, o.y, o.z, W.o[lane].w);
           if (!ok) *err = 1;
         }
-        if (ok && ref_is_node(R.ref) && !(S.has_motion && ref_is_frame(R.ref))) {
+        if (ok && ref_is_node(R.ref) && !(MOTION && ref_is_frame(R.ref))) {
           ok = visit_node<MODE != TRACE_ANY>(S, R, K);
           if (!ok) *err = 1;
         }
@@ -554,8 +605,9 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           R.sp = 0;
         }
       }
-      continue;
+      if (__popc(rm) <= walk_min) break;
     }
+    if (rm && qn < full) continue;
     if (!qn) {
       if (exhausted && idle == 0xffffffffu) break;
       continue;
@@ -580,7 +632,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
       const int32_t code = ~lref;  // first_item << 3 | count - 1
       const int last = (code >> 3) + (code & 7);
       for (int i = code >> 3; i <= last; ++i) {
-        if (test_item<CURVES>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w)) {
+        if (test_item<CURVES, MOTION>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w)) {
           hit = true;
           if (eany) break;
           tm = h.t;

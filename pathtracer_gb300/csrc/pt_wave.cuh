@@ -311,12 +311,11 @@ __global__ void k_camera(DeviceJob J0, JobTable T, Queues Q, long long g0, int n
 }
 
 // Free lanes (of 32) at which a traversal warp claims new rays (trace_rays).
-// Closest hits at 8 / 16 / 24: rough glass trace 14.1 / 13.75 / 13.5 ms,
-// Cornell 3.27 / 3.19 / 3.26.  Shadow rays at 8 / 16 / 24: rough glass 13.6 /
-// 13.3 / 14.1 ms, Cornell 7.3 / 6.66 / 6.83, material divergence 31.6 / 31.7 /
-// 34.3.
-#define PT_FETCH_IDLE 16
-#define PT_FETCH_IDLE_SHADOW 16
+// Both at 12 / 16 / 20: rough glass trace 11.1 / 11.4 / 11.3 ms and shadow 9.9 /
+// 10.2 / 10.9, Cornell trace 2.92 / 2.92 / 2.91 and shadow 6.97 / 6.90 / 6.77,
+// material divergence shadow 26.9 / 26.9 / 27.7.
+#define PT_FETCH_IDLE 12
+#define PT_FETCH_IDLE_SHADOW 12
 
 // k_trace_closest: the RayQueue through the BVH.  In a participating medium
 // the free-flight distance of the segment is drawn when the ray is fetched
@@ -351,12 +350,12 @@ __device__ __forceinline__ void store_closest(const Queues &Q, int r, bool found
   const float t = found ? h.t : (prim == PT_HIT_MEDIUM ? t_s : FLT_MAX);
   Q.hit[r] = make_float4(t, __int_as_float(prim), found ? h.u : 0.f, found ? h.v : 0.f);
 }
-template <bool MJ, bool CURVES>
+template <bool MJ, bool CURVES, bool MOTION>
 __device__ __forceinline__ void trace_closest_body(const SceneView &S, const DeviceJob &J, const JobTable &T,
                                                    const Queues &Q, int qsel, int bounce, long long g0, char *smem) {
   int ray = 0, rays = 0;
   float t_s = INFINITY;
-  trace_rays<TRACE_CLOSEST, CURVES>(
+  trace_rays<TRACE_CLOSEST, CURVES, MOTION>(
       S, Q.counts[qsel], Q.counts + 4, PT_FETCH_IDLE, Q.err, smem,
       [&](int r, V3 &o, V3 &d, float &tmin, float &tmax, float &time, bool &) {
         fetch_closest<MJ>(S, J, T, Q, qsel, bounce, g0, r, o, d, tmin, tmax, time, t_s);
@@ -370,11 +369,11 @@ __device__ __forceinline__ void trace_closest_body(const SceneView &S, const Dev
 // 8 resident blocks (64 registers): the unbounded 72 registers run 7 here and,
 // with one grid for both, 7 of the shadow kernel: Cornell shadow 7.8 -> 7.3 ms,
 // divergence 33.3 -> 31.7.
-template <bool MJ, bool CURVES>
-__global__ void __launch_bounds__(128, 8) k_trace_closest(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel,
+template <bool MJ, bool CURVES, bool MOTION>
+__global__ void __launch_bounds__(128, CURVES ? 6 : 8) k_trace_closest(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel,
                                                        int bounce, long long g0) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
-  trace_closest_body<MJ, CURVES>(S, J, T, Q, qsel, bounce, g0, smem);
+  trace_closest_body<MJ, CURVES, MOTION>(S, J, T, Q, qsel, bounce, g0, smem);
 }
 
 // k_trace_pair: the closest-hit rays of bounce `bounce` (RayQueue qsel)
@@ -400,7 +399,7 @@ __device__ __forceinline__ size_t fetch_shadow(const SceneView &S, const Queues 
   tmax = dd.w;
   return slot;
 }
-template <bool MJ, bool CURVES>
+template <bool MJ, bool CURVES, bool MOTION>
 __device__ __forceinline__ void trace_pair_body(const SceneView &S, const DeviceJob &J, const JobTable &T,
                                                 const Queues &Q, int qsel, int bounce, long long g0, char *smem) {
   const int nc = Q.counts[qsel];
@@ -408,7 +407,7 @@ __device__ __forceinline__ void trace_pair_body(const SceneView &S, const Device
   bool shadow = false;
   int crays = 0, srays = 0;
   float t_s = INFINITY;
-  trace_rays<TRACE_MIXED, CURVES>(
+  trace_rays<TRACE_MIXED, CURVES, MOTION>(
       S, nc + Q.counts[5], Q.counts + 4, PT_FETCH_IDLE, Q.err, smem,
       [&](int r, V3 &o, V3 &d, float &tmin, float &tmax, float &time, bool &any) {
         any = shadow = r >= nc;
@@ -429,11 +428,11 @@ __device__ __forceinline__ void trace_pair_body(const SceneView &S, const Device
   warp_count(&Q.stats[2], crays);
   warp_count(&Q.stats[3], srays);
 }
-template <bool MJ, bool CURVES>
+template <bool MJ, bool CURVES, bool MOTION>
 __global__ void __launch_bounds__(128, 7) k_trace_pair(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel,
                                                     int bounce, long long g0) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
-  trace_pair_body<MJ, CURVES>(S, J, T, Q, qsel, bounce, g0, smem);
+  trace_pair_body<MJ, CURVES, MOTION>(S, J, T, Q, qsel, bounce, g0, smem);
 }
 
 // The hit point in its object's rest frame (texture coordinates of moving
@@ -922,11 +921,11 @@ __global__ void __launch_bounds__(128, shade_min_blocks(FAM, MJ)) k_shade(SceneV
 // k_trace_closest.  Each ray's visibility goes to Q.sh_vis; k_shadow_resolve
 // then adds the visible terms of every vertex to its path in a fixed order,
 // so the result does not depend on which warp traced which ray.
-template <bool CURVES>
+template <bool CURVES, bool MOTION>
 __device__ __forceinline__ void trace_shadow_body(const SceneView &S, const Queues &Q, char *smem) {
   size_t slot = 0;
   int rays = 0;
-  trace_rays<TRACE_ANY, CURVES>(
+  trace_rays<TRACE_ANY, CURVES, MOTION>(
       S, Q.counts[5], Q.counts + 3, PT_FETCH_IDLE_SHADOW, Q.err, smem,
       [&](int r, V3 &o, V3 &d, float &tmin, float &tmax, float &time, bool &) {
         slot = fetch_shadow(S, Q, r, o, d, tmin, tmax, time);
@@ -1033,14 +1032,15 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
     P.begin(STAGE_TRACE, st);
     if (pair) {
       // this bounce's closest rays with the previous bounce's shadow rays
-      if (S.curves)
-        k_trace_pair<MJ, true><<<cfg.trace_blocks, 128, trace_smem(S, 128), st>>>(S, J, T, Q, qsel, b, g0);
-      else
-        k_trace_pair<MJ, false><<<cfg.trace_blocks, 128, trace_smem(S, 128), st>>>(S, J, T, Q, qsel, b, g0);
-    } else if (S.curves) {
-      k_trace_closest<MJ, true><<<cfg.trace_blocks, 128, trace_smem(S, 128), st>>>(S, J, T, Q, qsel, b, g0);
+#define PT_RUN(C, M) \
+  k_trace_pair<MJ, C, M><<<cfg.trace_blocks, 128, trace_smem(128), st>>>(S, J, T, Q, qsel, b, g0)
+      PT_BY_SCENE(S, PT_RUN);
+#undef PT_RUN
     } else {
-      k_trace_closest<MJ, false><<<cfg.trace_blocks, 128, trace_smem(S, 128), st>>>(S, J, T, Q, qsel, b, g0);
+#define PT_RUN(C, M) \
+  k_trace_closest<MJ, C, M><<<cfg.trace_blocks, 128, trace_smem(128), st>>>(S, J, T, Q, qsel, b, g0)
+      PT_BY_SCENE(S, PT_RUN);
+#undef PT_RUN
     }
     P.end(st);
     P.count(STAGE_TRACE, 1);
