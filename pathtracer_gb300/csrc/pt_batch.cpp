@@ -97,6 +97,8 @@ void BatchSlot::ensure(int want_cap, int want_ln, int n_jobs, size_t n_offsets, 
       Q.err = (int *)alloc(16);
       Q.sort_key = (int *)alloc(c * 4);
       Q.order = (int *)alloc(c * 4);
+      Q.smp = (float *)alloc(c * 12);
+      Q.smp_key = (uint64_t *)alloc(c * 8);
       Q.job = (int *)alloc(c * 4);
       Q.bins = (int *)alloc(sizeof(int) * 2 * PT_SORT_BINS);
       Q.seg = (int *)alloc(sizeof(int) * (PT_SORT_BINS + 1));

@@ -216,7 +216,8 @@ PT_HD uint64_t splitmix64(uint64_t z) {
 }
 PT_HD float rand01(uint64_t key, uint32_t slot) {
   uint64_t h = splitmix64(key ^ ((uint64_t)slot * 0xd1b54a32d192ed03ull));
-  return (float)(h >> 40) * (1.0f / 16777216.0f);
+  // 24 bits: converted from 32 (a 64-bit conversion runs on the FP64 pipe)
+  return (float)(uint32_t)(h >> 40) * (1.0f / 16777216.0f);
 }
 PT_HD uint64_t path_key(uint32_t seed, uint64_t sample_id) {
   return splitmix64(((uint64_t)seed << 40) ^ sample_id);
@@ -228,6 +229,10 @@ PT_HD uint64_t path_key(uint32_t seed, uint64_t sample_id) {
 // dim >= 25; this build defines it as Primes[dim % 25], the rule the
 // unscrambled radicalInverse already uses (utility.hpp:408).
 #define PT_PRIME_COUNT 25
+// Dimensions whose first Owen-scrambled digits are tabulated, and the largest
+// table's entries.
+#define PT_OWEN_DIMS 64
+#define PT_OWEN_ENTRIES (1u << 17)
 struct HaltonTables {
   int32_t prime[PT_PRIME_COUNT];
   int32_t ndigits[PT_PRIME_COUNT];    // digits visited by the double loop test
@@ -238,9 +243,17 @@ struct HaltonTables {
   uint32_t div_magic[PT_PRIME_COUNT];
   int32_t div_shift[PT_PRIME_COUNT];  // shift; bit 6 set: the 33-bit (add) form
   // Owen-scrambled digits after which the value is tested for being settled
-  // (the least k with prime^k >= 2^38), and prime^(ndigits - owen_check)
+  // (the least k with prime^k >= 2^35), and prime^(ndigits - owen_check)
   int32_t owen_check[PT_PRIME_COUNT];
   uint64_t owen_tail[PT_PRIME_COUNT];
+  // Tables of the first Owen-scrambled digits (owen_radical_inverse): the
+  // digits they cover, prime^digits with its division, and where dimension d's
+  // table begins
+  int32_t owen_first[PT_PRIME_COUNT];
+  uint32_t owen_pow[PT_PRIME_COUNT];
+  uint32_t owen_pow_magic[PT_PRIME_COUNT];
+  int32_t owen_pow_shift[PT_PRIME_COUNT];
+  uint32_t owen_at[PT_OWEN_DIMS + 1];
 };
 
 // The magic multiplier and shift of a / d for every 32-bit a (d >= 2):
@@ -268,10 +281,8 @@ inline void div_invariant(uint32_t d, uint32_t &magic, int32_t &shift) {
   magic = m + 1;
 }
 
-// a / T.prime[bi] for every 32-bit a.
-PT_HD uint32_t div_prime(const HaltonTables &T, int bi, uint32_t a) {
-  const uint32_t m = T.div_magic[bi];
-  const int s = T.div_shift[bi];
+// a / d for every 32-bit a by d's magic multiplier m and shift s.
+PT_HD uint32_t div_by(uint32_t m, int s, uint32_t a) {
   if (!m) return a >> s;
 #ifdef __CUDA_ARCH__
   const uint32_t q = __umulhi(m, a);
@@ -280,6 +291,10 @@ PT_HD uint32_t div_prime(const HaltonTables &T, int bi, uint32_t a) {
 #endif
   if (s & 64) return (((a - q) >> 1) + q) >> (s & 63);
   return q >> s;
+}
+// a / T.prime[bi].
+PT_HD uint32_t div_prime(const HaltonTables &T, int bi, uint32_t a) {
+  return div_by(T.div_magic[bi], T.div_shift[bi], a);
 }
 
 // gl::radicalInverse (utility.hpp:406-420), float arithmetic.
@@ -315,7 +330,7 @@ PT_HD float clamp_to_float(double r) {
 // the first k can only place rev in [rev_k * b^r, rev_k * b^r + b^r - 1]
 // (r = ndigits - k).  Where f takes the same value at both ends, that is
 // the result whatever the remaining digits are, so the loop stops there;
-// after T.owen_check digits this settles all but a few in 10^4 samples
+// after T.owen_check digits this settles all but a few in 10^3 samples
 // (the rest run every digit as the reference does).
 struct OwenDigits {
   uint32_t a;    // the index's digits not yet taken
@@ -342,14 +357,23 @@ PT_HD void owen_digit(const HaltonTables &T, int bi, uint32_t base, uint32_t w, 
     s.a = next;
   }
 }
+// The scrambled digits of the first T.owen_first digits depend on the index
+// modulo T.owen_pow only: `first`, the dimension's table by that remainder (or
+// null), gives them with one load in place of 2 (base 97) to 17 (base 2) of the
+// 6 to 38 digits up to the early end.
 template <bool BASE2>
-PT_HD float owen_digits(const HaltonTables &T, int bi, uint32_t hash, uint32_t index) {
+PT_HD float owen_digits(const HaltonTables &T, int bi, uint32_t hash, uint32_t index, const uint32_t *first) {
   const uint32_t base = (uint32_t)T.prime[bi];
   const uint32_t w = fill_mask(base);
   const double scale = T.inv_base_m[bi];
   OwenDigits s{index, 0};
   const int nd = T.ndigits[bi], nc = T.owen_check[bi];
   int di = 0;
+  if (first) {
+    s.a = div_by(T.owen_pow_magic[bi], T.owen_pow_shift[bi], index);
+    s.rev = first[index - s.a * T.owen_pow[bi]];
+    di = T.owen_first[bi];
+  }
   for (; di < nc; ++di) owen_digit<BASE2>(T, bi, base, w, hash, di, s);
   const uint64_t lo = s.rev * T.owen_tail[bi];
   const float flo = clamp_to_float(xdmul(scale, (double)lo));
@@ -357,10 +381,44 @@ PT_HD float owen_digits(const HaltonTables &T, int bi, uint32_t hash, uint32_t i
   for (; di < nd; ++di) owen_digit<BASE2>(T, bi, base, w, hash, di, s);
   return clamp_to_float(xdmul(scale, (double)s.rev));
 }
-PT_HD float owen_radical_inverse(const HaltonTables &T, int dim, uint32_t index) {
+// The scrambling of dimension dim (sampler.hpp:69-71).
+PT_HD uint32_t owen_hash(int dim) { return (uint32_t)mix_bits(1u + ((uint32_t)dim << 4)); }
+// `tables`: the first digits of dimensions 0..PT_OWEN_DIMS-1 (T.owen_at), or
+// null.
+PT_HD float owen_radical_inverse(const HaltonTables &T, int dim, uint32_t index, const uint32_t *tables = nullptr) {
   const int bi = dim % PT_PRIME_COUNT;
-  const uint32_t hash = (uint32_t)mix_bits(1u + ((uint32_t)dim << 4));
-  return T.prime[bi] == 2 ? owen_digits<true>(T, bi, hash, index) : owen_digits<false>(T, bi, hash, index);
+  const uint32_t hash = owen_hash(dim);
+  const uint32_t *first = tables && dim < PT_OWEN_DIMS ? tables + T.owen_at[dim] : nullptr;
+  return T.prime[bi] == 2 ? owen_digits<true>(T, bi, hash, index, first)
+                          : owen_digits<false>(T, bi, hash, index, first);
+}
+// Entry r of dimension dim's table.
+PT_HD uint32_t owen_first_digits(const HaltonTables &T, int dim, uint32_t r) {
+  const int bi = dim % PT_PRIME_COUNT;
+  const uint32_t base = (uint32_t)T.prime[bi], w = fill_mask(base), hash = owen_hash(dim);
+  OwenDigits s{r, 0};
+  for (int di = 0; di < T.owen_first[bi]; ++di) {
+    if (base == 2) owen_digit<true>(T, bi, base, w, hash, di, s);
+    else owen_digit<false>(T, bi, base, w, hash, di, s);
+  }
+  return (uint32_t)s.rev;
+}
+// The tables' layout in T; returns their entries in all.
+inline uint32_t owen_table_layout(HaltonTables &T) {
+  for (int b = 0; b < PT_PRIME_COUNT; ++b) {
+    uint32_t pow = 1;
+    int digits = 0;
+    while (pow * (uint32_t)T.prime[b] <= PT_OWEN_ENTRIES) {
+      pow *= (uint32_t)T.prime[b];
+      ++digits;
+    }
+    T.owen_first[b] = digits;
+    T.owen_pow[b] = pow;
+    div_invariant(pow, T.owen_pow_magic[b], T.owen_pow_shift[b]);
+  }
+  T.owen_at[0] = 0;
+  for (int d = 0; d < PT_OWEN_DIMS; ++d) T.owen_at[d + 1] = T.owen_at[d] + T.owen_pow[d % PT_PRIME_COUNT];
+  return T.owen_at[PT_OWEN_DIMS];
 }
 
 // gl::scrambledRadicalInverse with DigitPermutation tables

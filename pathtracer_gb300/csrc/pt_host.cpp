@@ -59,12 +59,13 @@ HaltonTables make_halton_tables() {
     off += nd * base;
     div_invariant((uint32_t)base, T.div_magic[b], T.div_shift[b]);
     int check = 0;
-    for (uint64_t p = 1; p < (1ull << 38) && check < nd; p *= (uint64_t)base) ++check;
+    for (uint64_t p = 1; p < (1ull << 35) && check < nd; p *= (uint64_t)base) ++check;
     uint64_t tail = 1;
     for (int r = check; r < nd; ++r) tail *= (uint64_t)base;
     T.owen_check[b] = check;
     T.owen_tail[b] = tail;
   }
+  owen_table_layout(T);
   return T;
 }
 
@@ -1614,6 +1615,8 @@ Context::Context(int dev) : device(dev) {
   upload_halton_tables(halton, stream);
   upload_halton_tables_multi(halton, stream);
   upload_halton_tables_persist(halton, stream);
+  cuda_check(cudaMalloc(&d_owen, sizeof(uint32_t) * halton.owen_at[PT_OWEN_DIMS]), "cudaMalloc(owen tables)");
+  launch_owen_tables(d_owen, halton.owen_at[PT_OWEN_DIMS], stream);
   kernel_attributes(&kinfo);
   cfg.trace_blocks = num_sms * std::max(1, kinfo.trace_blocks_per_sm);
   cfg.shade_blocks = num_sms * std::max(1, kinfo.shade_blocks_per_sm);
@@ -1661,6 +1664,7 @@ Context::~Context() {
   if (d_offsets) cudaFree(d_offsets);
   if (d_scratch) cudaFree(d_scratch);
   if (d_err) cudaFree(d_err);
+  if (d_owen) cudaFree(d_owen);
   for (cudaEvent_t e : prof.pool) cudaEventDestroy(e);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -1700,6 +1704,8 @@ static void alloc_queues(Queues &Q, std::vector<void *> &mem, int cap, int ln, i
   Q.stats = (unsigned long long *)alloc(64);
   Q.sort_key = (int *)alloc(c * 4);
   Q.order = (int *)alloc(c * 4);
+  Q.smp = (float *)alloc(c * 12);
+  Q.smp_key = (uint64_t *)alloc(c * 8);
   Q.bins = (int *)alloc(sizeof(int) * 2 * PT_SORT_BINS);
   Q.seg = (int *)alloc(sizeof(int) * (PT_SORT_BINS + 1));
   Q.job = (int *)alloc(c * 4);
@@ -1839,6 +1845,7 @@ DeviceJob Context::device_job(const pt_job_desc &j, Scene *S) {
   J.job.seed = j.seed;
   J.job.shutter = j.camera.shutter;
   J.job.cam = make_camera(j.camera);
+  J.owen = d_owen;
   J.perm = j.sampler == PT_SAMPLER_HALTON_PERMUTE ? perm_for(j.sampler_seed) : nullptr;
   if (S->view.has_motion && j.camera.shutter > S->shutter_max)
     fail(PT_ERR_INVALID, "camera shutter longer than the scene's shutter_max");

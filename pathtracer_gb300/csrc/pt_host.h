@@ -134,6 +134,7 @@ struct Context {
   int offsets_cap = 0;
   void *d_scratch = nullptr;
   size_t scratch_cap = 0;
+  uint32_t *d_owen = nullptr;  // first digits of the Owen-scrambled dimensions (11 MB, as long as the context)
   int *d_err = nullptr;    // device error flag
   int *d_fetch = nullptr;  // fetch counter of the ray-query kernels (behind d_err)
   Profiler prof;

@@ -366,6 +366,19 @@ __global__ void k_tonemap(const float *film, int W, int H, float inv_gamma, uint
   }
 }
 
+// The tables of first Owen-scrambled digits, one entry per thread (a context's
+// creation).
+__global__ void k_owen_tables(uint32_t *tables, uint32_t n) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    int dim = 0;
+    while (c_halton.owen_at[dim + 1] <= i) ++dim;
+    tables[i] = owen_first_digits(c_halton, dim, i - c_halton.owen_at[dim]);
+  }
+}
+void launch_owen_tables(uint32_t *tables, uint32_t n, cudaStream_t st) {
+  k_owen_tables<<<grid_for(n, 256, 152 * 16), 256, 0, st>>>(tables, n);
+}
+
 // The traversal's nodes from the built ones, one per thread (a scene upload).
 __global__ void k_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = pack_node(nodes[i]);
@@ -494,14 +507,14 @@ void kernel_attributes(KernelInfo *info) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_trace_shadow<false, false>, 128, smax);
   info->shadow_blocks_per_sm = nb;
   int *fb = info->shade_fam_blocks_per_sm;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[0], k_shade<0, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[1], k_shade<1, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[2], k_shade<2, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[3], k_shade<3, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[4], k_shade<4, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[5], k_shade<5, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[6], k_shade<6, false>, 128, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[PT_FAM_MISC], k_shade<PT_FAM_MISC, false>, 128, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[0], k_shade<0, false>, shade_threads(0), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[1], k_shade<1, false>, shade_threads(1), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[2], k_shade<2, false>, shade_threads(2), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[3], k_shade<3, false>, shade_threads(3), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[4], k_shade<4, false>, shade_threads(4), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[5], k_shade<5, false>, shade_threads(5), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[6], k_shade<6, false>, shade_threads(6), 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fb[PT_FAM_MISC], k_shade<PT_FAM_MISC, false>, shade_threads(PT_FAM_MISC), 0);
   fb[PT_FAM_MISC + 1] = info->shade_blocks_per_sm;
 }
 

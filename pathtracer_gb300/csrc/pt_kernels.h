@@ -24,6 +24,7 @@ namespace pt {
 struct DeviceJob {
   JobView job;
   const uint16_t *perm;  // PermuteDigits tables for job.sampler_seed
+  const uint32_t *owen;  // the context's tables of first Owen-scrambled digits
 };
 
 // Jobs of a merged wave (batched and served forms): the merged path index
@@ -52,6 +53,8 @@ struct Queues {
   int *err;           // device error flag (stack overflow / iteration cap)
   int *job;           // [cap] merged waves: job index of the path in each slot
   int *sort_key, *order, *bins;
+  float *smp;         // [3][cap]: the sampler dimensions of the sorted queue's vertices (k_sample)
+  uint64_t *smp_key;  // [cap]: and their counter-stream keys
   int *seg;           // [PT_SORT_BINS + 1] segment bounds of the sorted order
 };
 
@@ -136,6 +139,7 @@ struct KernelInfo {
 };
 
 void upload_halton_tables(const HaltonTables &T, cudaStream_t st);
+void launch_owen_tables(uint32_t *tables, uint32_t n, cudaStream_t st);
 void launch_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out, cudaStream_t st);
 void launch_light_eval(const SceneView &S, int light, int n, const float *uv, const float *x, const float *pdf_dir,
                        float *point, float *normal, float *dir, float *le, float *pdf, cudaStream_t st);

@@ -96,8 +96,8 @@ __device__ __noinline__ void st_trace(const SceneView &S, const DeviceJob &none,
     trace_closest_body<true, CURVES, MOTION>(S, none, T, Q, qsel, b, g0, smem);
 }
 __device__ __noinline__ void st_shade(const SceneView &S, const DeviceJob &none, const JobTable &T, const Queues &Q,
-                                      int qsel, int b, long long g0) {
-  shade_body<-1, true>(S, none, T, Q, qsel, b, g0);
+                                      int qsel, int b, long long g0, int LN) {
+  shade_body<-1, true>(S, none, T, Q, qsel, b, g0, LN);
 }
 template <bool CURVES, bool MOTION>
 __device__ __noinline__ void st_shadow(const SceneView &S, const Queues &Q, char *smem) {
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(PT_PERSIST_THREADS, PT_PERSIST_MIN_BLOCKS)
         shadow_resolve_body(Q, LN);
         if (!grid_sync(bar, [=] { cnt[2] = 0; cnt[3] = 0; cnt[5] = 0; })) return;
       }
-      st_shade(S, none, T, Q, qsel, b, g0);
+      st_shade(S, none, T, Q, qsel, b, g0, LN);
       if (!grid_sync(bar, NoReset())) return;
       qsel = nq;
     }

@@ -82,8 +82,8 @@ void render_device_noalloc(Context *c, const pt_job_desc &j, float *d_film, pt_s
   uint16_t *d_perm = (uint16_t *)carve(perm.size() * sizeof(uint16_t) + 16);
   const int LN = j.light_samples_x * j.light_samples_y;
   off = align_up(off, 256);
-  const size_t per_path = 16 * 8 + 2 * 16 * (size_t)LN + 5 * (size_t)LN + 3 * 4;
-  const size_t avail = PT_NOALLOC_SCRATCH_BYTES - off - 19 * 256;  // alignment slack of 19 arrays
+  const size_t per_path = 16 * 8 + 2 * 16 * (size_t)LN + 5 * (size_t)LN + 3 * 4 + 20;
+  const size_t avail = PT_NOALLOC_SCRATCH_BYTES - off - 21 * 256;  // alignment slack of 21 arrays
   const int cap = (int)std::min<size_t>(avail / per_path, (size_t)1 << 30);
   if (cap < 1024) fail(PT_ERR_TOO_LARGE, "pt_render_device_noalloc: scratch too small for the light samples");
   const size_t c4 = (size_t)cap * 16;
@@ -102,6 +102,8 @@ void render_device_noalloc(Context *c, const pt_job_desc &j, float *d_film, pt_s
   Q.sh_list = (uint32_t *)carve((size_t)cap * LN * 4);
   Q.sort_key = (int *)carve((size_t)cap * 4);
   Q.order = (int *)carve((size_t)cap * 4);
+  Q.smp = (float *)carve((size_t)cap * 12);
+  Q.smp_key = (uint64_t *)carve((size_t)cap * 8);
   Q.job = (int *)carve((size_t)cap * 4);
   if (off > PT_NOALLOC_SCRATCH_BYTES) fail(PT_ERR_TOO_LARGE, "pt_render_device_noalloc: scratch layout overflow");
 
@@ -125,6 +127,7 @@ void render_device_noalloc(Context *c, const pt_job_desc &j, float *d_film, pt_s
   if (S->view.has_motion && j.camera.shutter > S->shutter_max)
     fail(PT_ERR_INVALID, "camera shutter longer than the scene's shutter_max");
   J.job.cam = make_camera(j.camera);
+  J.owen = c->d_owen;
   std::vector<float2> offs = make_offsets(j);
   cuda_check(cudaMemcpyAsync(d_off, offs.data(), offs.size() * sizeof(float2), cudaMemcpyHostToDevice, c->stream),
              "upload offsets");

@@ -34,6 +34,7 @@ __device__ __forceinline__ uint32_t ldu(const uint32_t *p) { return __ldcg(p); }
 __device__ __forceinline__ float4 ld4(const float4 *p) { return __ldg(p); }
 __device__ __forceinline__ uint32_t ldu(const uint32_t *p) { return __ldg(p); }
 #endif
+__device__ __forceinline__ float ldf(const float *p) { return __ldg(p); }
 
 // Warp-aggregated slot allocation in a queue counter.
 __device__ __forceinline__ int warp_alloc(int *counter, bool want) {
@@ -66,7 +67,7 @@ __device__ __forceinline__ float sampler_dim(const DeviceJob &J, int dim, uint32
     float jit = rand01(key, 4096u + (uint32_t)dim);
     return fminf(((float)stratum + jit) / (float)S, 0x1.fffffep-1f);
   }
-  default: return owen_radical_inverse(c_halton, dim, index);
+  default: return owen_radical_inverse(c_halton, dim, index, J.owen);
   }
 }
 
@@ -220,8 +221,14 @@ struct PathId {
 __device__ __forceinline__ PathId path_id(const DeviceJob &J, long long g) {
   PathId P;
   const long long npix = (long long)J.job.width * J.job.height;
-  P.q = (int)(g % npix);
-  P.k = J.job.spp_begin + (int)(g / npix);
+  if (((unsigned long long)g >> 32) == 0) {  // a 64-bit division takes ~4x the instructions
+    const uint32_t g32 = (uint32_t)g, n32 = (uint32_t)npix, plane = g32 / n32;
+    P.q = (int)(g32 - plane * n32);
+    P.k = J.job.spp_begin + (int)plane;
+  } else {
+    P.q = (int)(g % npix);
+    P.k = J.job.spp_begin + (int)(g / npix);
+  }
   P.i = J.job.crop_x + P.q % J.job.width;
   P.j = J.job.crop_y + P.q / J.job.width;
   P.pix = P.j * J.job.full_w + P.i;
@@ -568,23 +575,21 @@ __device__ inline float light_pdf_value(const LightRec &Lr, V3 origin, V3 dir) {
   return dist2 / (Lr.area * cos_t);
 }
 
-// Next-event estimation at one vertex (maxdepth_nee.hpp:89-232): LN light
-// samples on a stratified x-by-y grid, each a ShadowQueue entry with its
-// unoccluded contribution.  Returns the samples that contribute (bit ls); the
-// others are marked invisible and write no record.  MED: the vertex is a medium scattering event
+// Next-event estimation at one vertex (maxdepth_nee.hpp:89-232): light sample
+// ls of the LN on a stratified x-by-y grid, a ShadowQueue entry with its
+// unoccluded contribution.  Returns whether it contributes; if not it is
+// marked invisible and writes no record.  MED: the vertex is a medium scattering event
 // (isotropic phase function instead of a BSDF, no surface cosine).
 template <int FAM, bool MED>
-__device__ __forceinline__ unsigned next_event(const SceneView &S, const DeviceJob &J, const Queues &Q, int sslot,
-                                               int path, uint64_t key, uint32_t rbase, const Surf &sf, int mat,
-                                               V3 wo, V3 beta, int LN, bool mis, float time, bool tex_alb,
+__device__ __forceinline__ bool next_event(const SceneView &S, const DeviceJob &J, const Queues &Q, int sslot,
+                                               uint64_t key, uint32_t rbase, const Surf &sf, int mat,
+                                               V3 wo, V3 beta, int LN, int ls, bool mis, float time, bool tex_alb,
                                                V3 alb) {
-  unsigned lit = 0;
   const float phase = (float)(1.0 / (4.0 * PT_PI));
-  Q.sh_o[sslot] = make_float4(sf.p.x, sf.p.y, sf.p.z, __int_as_float(path));
   const float inv_ln = 1.f / (float)LN;
   const bool med = S.has_medium != 0;
-  for (int ls = 0; ls < LN; ++ls) {
-    bool contributes = false;
+  bool contributes = false;
+  {
     const float2 lo = light_offset(J, key, rbase, ls);
     const float ox = lo.x, oy = lo.y;
     int li = (int)(rand01(key, rbase + 20u + ls) * S.n_lights) % S.n_lights;
@@ -653,10 +658,9 @@ __device__ __forceinline__ unsigned next_event(const SceneView &S, const DeviceJ
         }
       }
     }
-    if (contributes) lit |= 1u << ls;
-    else Q.sh_vis[(size_t)ls * Q.cap + sslot] = 0;
   }
-  return lit;
+  if (!contributes) Q.sh_vis[(size_t)ls * Q.cap + sslot] = 0;
+  return contributes;
 }
 
 // The warp's contributing light samples (bit ls of `lit`, vertex sslot) go to
@@ -682,6 +686,37 @@ __device__ __forceinline__ void list_shadow_rays(const Queues &Q, unsigned lit, 
   }
 }
 
+// k_sample: the sampler dimensions of the sorted queue's vertices (three of a
+// surface's, two of a medium event's), one per thread, and the vertices'
+// counter-stream keys, for the per-family shade kernels.  Bound by the integer
+// pipe (76 % busy).  It takes 17-57 KB of sampler code out of each family's
+// kernel and runs it at 3 times their occupancy; with the tables of first
+// digits (owen_digits) rough glass shades 16.8 M paths in 13.1 ms instead of
+// 15.0, the Cornell frame in 6.2 instead of 7.3 (2^15 / 2^20 entries per table:
+// 13.4 / 12.8 ms; 2^17 keeps all 64 tables at 12 MB), and 12.9 / 6.0 with the
+// early end tested from b^k >= 2^35 instead of 2^38.
+template <bool MJ>
+__global__ void __launch_bounds__(256) k_sample(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel, int bounce,
+                                                long long g0) {
+  const int ns = Q.seg[PT_FAM_MISC], m0 = Q.seg[PT_KEY_MEDIUM], nm = Q.seg[PT_KEY_MEDIUM + 1] - m0;
+  const bool med = S.has_medium != 0;
+  const int first = (med ? 4 : 3) * bounce;  // the bounce's first dimension
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * ns + 2 * nm; t += gridDim.x * blockDim.x) {
+    const bool surf = t < 3 * ns;
+    const int u = surf ? t : t - 3 * ns, n = surf ? ns : nm;
+    const int d = (u >= n) + (surf && u >= 2 * n);
+    const int ii = u - d * n + (surf ? 0 : m0);
+    const int path = __float_as_int(ld4(Q.ray_o[qsel] + Q.order[ii]).w);
+    long long g;
+    const DeviceJob &Jp = path_job<MJ>(J, T, Q, path, g0, g);
+    if (bounce >= Jp.job.max_depth) continue;  // nothing is sampled there
+    const PathId P = path_id(Jp, g);
+    const int dim = first + (surf ? (med ? 1 : 0) : 2) + d;
+    Q.smp[(size_t)d * Q.cap + ii] = sampler_dim(Jp, dim, P.halton_index, P.key, P.pix, P.k);
+    if (d == 0) Q.smp_key[ii] = P.key;
+  }
+}
+
 // k_shade<FAM>: one path vertex per thread.  FAM 0..6 processes the
 // material-sorted segment of that BSDF family with its code compiled alone;
 // FAM PT_FAM_MISC the misses, emitter hits and medium events; FAM -1 the
@@ -697,19 +732,36 @@ __device__ __forceinline__ void list_shadow_rays(const Queues &Q, unsigned lit, 
 // NEE_MIS weights light and BSDF sampling with the power heuristic and
 // always performs NEE at non-delta vertices.  The loop runs in phases so
 // that the queue slot allocations (warp ballots) see every lane.
-// Resident blocks per SM a shade kernel is compiled for: families whose BSDF
-// code fits 102 registers without spilling run 5 blocks of 128 threads per
-// SM (the compiler's default allocation gave them 96-128 registers, 4-5
-// blocks); the Disney and hair kernels and the generic one, which spill
-// below 128 registers, run 4.  Single-job and merged-wave variants get the
-// same bound: a tighter one (6 blocks, 80 registers) changes how the
-// compiler contracts multiply-adds, and the two variants must compute the
-// same bits (a batched job equals its plain render).
-constexpr int shade_min_blocks(int fam, bool) { return (fam == 5 || fam == 6 || fam < 0) ? 4 : 5; }
+//
+// Blocks.  A family's kernel is 60-370 KB of code, most of it run once per
+// vertex and light sample, so warps at different places of it miss the
+// instruction caches (the largest stall after fixed latencies: 2.6-4.3 of ~9
+// warps per issue, conductors to Disney).  The families with a BSDF worth the
+// name therefore run blocks as large as an SM's share of warps, with a barrier
+// before each round of vertices and each light sample: the block's warps run
+// the same code at the same time and share its fetches.  Rough glass, 16.8 M
+// paths: shade 18.4 -> 15.0 ms; material divergence, 8.3 M paths: 39.3 -> 24.6.
+// Two blocks of 320 threads against one of 640: 15.0 / 15.5 ms; Disney and hair
+// with one block of 512 against two of 256: 24.6 / 28.2; further barriers
+// (between light point and BSDF): no gain.  The Lambertian kernel (7.28 -> 7.67
+// ms on the Cornell box) and the misses, emitters and medium events (24.6 ->
+// 26.7) are slower with them and keep 128 threads.
+// Registers: 640 threads per SM leave 102 each; the Disney and hair kernels and
+// the generic one, which spill there, run 512 threads (128 registers).
+// Single-job and merged-wave variants get the same bound: a tighter one (80
+// registers) changes how the compiler contracts multiply-adds, and the two
+// variants must compute the same bits (a batched job equals its plain render).
+constexpr int shade_threads(int fam) {
+  return (fam <= 0 || fam == PT_FAM_MISC) ? 128 : (fam == 5 || fam == 6) ? 512 : 320;
+}
+constexpr int shade_min_blocks(int fam) {
+  return ((fam == 5 || fam == 6 || fam < 0) ? 512 : 640) / shade_threads(fam);
+}
+constexpr bool shade_sync(int fam) { return fam > 0 && fam != PT_FAM_MISC; }
 
 template <int FAM, bool MJ>
 __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &J, const JobTable &T, const Queues &Q,
-                                           int qsel, int bounce, long long g0) {
+                                           int qsel, int bounce, long long g0, int LN) {
   int lo = 0, hi = Q.counts[qsel];
   if (FAM >= 0) {
     lo = Q.seg[FAM];
@@ -726,7 +778,10 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
   int segs = 0;
   const int stride = gridDim.x * blockDim.x;
   const int nround = (n + stride - 1) / stride * stride;
-  for (int ii = blockIdx.x * blockDim.x + threadIdx.x; ii < nround; ii += stride) {
+  // consecutive warps of vertices go to consecutive blocks: a short queue is
+  // spread over the SMs
+  for (int ii = (blockIdx.x + gridDim.x * (threadIdx.x >> 5)) * 32 + (threadIdx.x & 31); ii < nround; ii += stride) {
+    if (shade_sync(FAM)) __syncthreads();
     // ---------------- phase A: hit logic and BSDF sampling
     bool do_nee = false, push = false, nee_medium = false;
     int path = 0, mat = 0;
@@ -738,7 +793,6 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
     float npdf = -1.f;
     uint64_t key = 0;
     float time = 0.f;
-    int LN = 1;
     bool mis = false;
     bool tex_alb = false;  // textured Lambertian albedo of this vertex
     V3 alb = v3(0.f);
@@ -754,12 +808,20 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
       const float prev_pdf = b4.w;  // < 0: camera ray or previous vertex delta
       long long g;
       const DeviceJob &Jp = path_job<MJ>(J, T, Q, path, g0, g);
-      LN = Jp.job.light_nx * Jp.job.light_ny;
       mis = Jp.job.estimator == PT_EST_NEE_MIS;
       const int max_depth = Jp.job.max_depth;
       const int limit = mis ? max_depth + 1 : max_depth;
-      PathId P = path_id(Jp, g);
-      key = P.key;
+      PathId P;
+      if (FAM < 0) {
+        P = path_id(Jp, g);
+        key = P.key;
+      }
+      // sampler dimension d of the vertex: k_sample's record, or drawn here by
+      // the generic kernel
+      auto draw = [&](int first, int d) {
+        return FAM < 0 ? sampler_dim(Jp, first + d, P.halton_index, P.key, P.pix, P.k)
+                       : ldf(Q.smp + (size_t)d * Q.cap + (lo + ii));
+      };
       const int prim = __float_as_int(hh.y);
       V3 Ladd = v3(0.f);
       if (med && bounce >= max_depth) beta = beta * expf(-S.sigma_t_max * (prim >= 0 ? hh.x : INFINITY));
@@ -771,9 +833,10 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
                          S.sigma_s[2] / (S.sigma_a[2] + S.sigma_s[2]));
         do_nee = S.n_lights > 0;
         nee_medium = true;
+        if (FAM >= 0) key = Q.smp_key[lo + ii];
         if (bounce + 1 < limit) {
-          float u0 = sampler_dim(Jp, dpb * bounce + 2, P.halton_index, P.key, P.pix, P.k);
-          float u1 = sampler_dim(Jp, dpb * bounce + 3, P.halton_index, P.key, P.pix, P.k);
+          float u0 = draw(dpb * bounce + 2, 0);
+          float u1 = draw(dpb * bounce + 2, 1);
           float z = 1.f - 2.f * u0, rr = sqrtf(fmaxf(0.f, 1.f - z * z));
           float sp, cp;
           sincospi_(2.f * u1, &sp, &cp);
@@ -834,9 +897,8 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
         } else if (DO_SURF && !mat_is_emitter(M) && bounce < max_depth) {
           ++segs;
           const int dim0 = dpb * bounce + (med ? 1 : 0);
-          float uc = sampler_dim(Jp, dim0, P.halton_index, P.key, P.pix, P.k);
-          float u0 = sampler_dim(Jp, dim0 + 1, P.halton_index, P.key, P.pix, P.k);
-          float u1 = sampler_dim(Jp, dim0 + 2, P.halton_index, P.key, P.pix, P.k);
+          if (FAM >= 0) key = Q.smp_key[lo + ii];
+          float uc = draw(dim0, 0), u0 = draw(dim0, 1), u1 = draw(dim0, 2);
           wo = -normalize(d);
           // HairMarschner::scatter on a curve samples the direction and its
           // pdf in the curve tangent's frame (hairMarsch.cpp:12-24) while its
@@ -876,7 +938,7 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
               if (Jp.job.rr_start >= 0 && bounce >= Jp.job.rr_start) {
                 // roulette_naive.hpp:35-38 applied to the continuation
                 float q = clampf(max_comp(bs.att), 0.5f, 1.0f);
-                if (rand01(P.key, rbase + 31u) > q) push = false;
+                if (rand01(key, rbase + 31u) > q) push = false;
                 nb = nb * (1.f / q);
               }
             }
@@ -898,22 +960,29 @@ __device__ __forceinline__ void shade_body(const SceneView &S, const DeviceJob &
     }
     // ---------------- phase C: next-event estimation
     unsigned lit = 0;
-    if (do_nee) {
-      long long g;
-      const DeviceJob &Jp = path_job<MJ>(J, T, Q, path, g0, g);
-      if (DO_MISC && nee_medium)
-        lit = next_event<FAM, true>(S, Jp, Q, sslot, path, key, rbase, sf, mat, wo, beta, LN, mis, time, false, alb);
-      else if (DO_SURF)
-        lit = next_event<FAM, false>(S, Jp, Q, sslot, path, key, rbase, sf, mat, wo, beta, LN, mis, time, tex_alb, alb);
+    if (do_nee) Q.sh_o[sslot] = make_float4(sf.p.x, sf.p.y, sf.p.z, __int_as_float(path));
+#pragma unroll 1
+    for (int ls = 0; ls < LN; ++ls) {
+      if (shade_sync(FAM)) __syncthreads();
+      if (do_nee) {
+        long long g;
+        const DeviceJob &Jp = path_job<MJ>(J, T, Q, path, g0, g);
+        bool c = false;
+        if (DO_MISC && nee_medium)
+          c = next_event<FAM, true>(S, Jp, Q, sslot, key, rbase, sf, mat, wo, beta, LN, ls, mis, time, false, alb);
+        else if (DO_SURF)
+          c = next_event<FAM, false>(S, Jp, Q, sslot, key, rbase, sf, mat, wo, beta, LN, ls, mis, time, tex_alb, alb);
+        lit |= (unsigned)c << ls;
+      }
     }
     list_shadow_rays(Q, lit, sslot);
   }
   warp_count(&Q.stats[1], segs);
 }
 template <int FAM, bool MJ>
-__global__ void __launch_bounds__(128, shade_min_blocks(FAM, MJ)) k_shade(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel, int bounce,
-                                               long long g0) {
-  shade_body<FAM, MJ>(S, J, T, Q, qsel, bounce, g0);
+__global__ void __launch_bounds__(shade_threads(FAM), shade_min_blocks(FAM)) k_shade(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel, int bounce,
+                                               long long g0, int LN) {
+  shade_body<FAM, MJ>(S, J, T, Q, qsel, bounce, g0, LN);
 }
 
 // k_trace_shadow: the listed rays of the ShadowQueue (vertex v, light sample
@@ -1059,6 +1128,10 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
       P.end(st);
       P.count(STAGE_SORT, 2);
       P.begin(STAGE_SHADE, st);
+      if (MJ || b < J.job.max_depth) {
+        k_sample<MJ><<<cfg.max_blocks_simple, 256, 0, st>>>(S, J, T, Q, qsel, b, g0);
+        P.count(STAGE_SHADE, 1);
+      }
       // the families present, then misses / emitters / medium events, each
       // on the next of the stream and its side streams (round robin)
       int used = 0;  // side streams forked
@@ -1074,14 +1147,14 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
         }
         return ss->aux[slot - 1];
       };
-      if (cfg.family_mask & (1u << 0)) k_shade<0, MJ><<<cfg.shade_fam_blocks[0], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      if (cfg.family_mask & (1u << 1)) k_shade<1, MJ><<<cfg.shade_fam_blocks[1], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      if (cfg.family_mask & (1u << 2)) k_shade<2, MJ><<<cfg.shade_fam_blocks[2], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      if (cfg.family_mask & (1u << 3)) k_shade<3, MJ><<<cfg.shade_fam_blocks[3], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      if (cfg.family_mask & (1u << 4)) k_shade<4, MJ><<<cfg.shade_fam_blocks[4], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      if (cfg.family_mask & (1u << 5)) k_shade<5, MJ><<<cfg.shade_fam_blocks[5], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      if (cfg.family_mask & (1u << 6)) k_shade<6, MJ><<<cfg.shade_fam_blocks[6], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
-      k_shade<PT_FAM_MISC, MJ><<<cfg.shade_fam_blocks[PT_FAM_MISC], 128, 0, next_stream()>>>(S, J, T, Q, qsel, b, g0);
+      if (cfg.family_mask & (1u << 0)) k_shade<0, MJ><<<cfg.shade_fam_blocks[0], shade_threads(0), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      if (cfg.family_mask & (1u << 1)) k_shade<1, MJ><<<cfg.shade_fam_blocks[1], shade_threads(1), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      if (cfg.family_mask & (1u << 2)) k_shade<2, MJ><<<cfg.shade_fam_blocks[2], shade_threads(2), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      if (cfg.family_mask & (1u << 3)) k_shade<3, MJ><<<cfg.shade_fam_blocks[3], shade_threads(3), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      if (cfg.family_mask & (1u << 4)) k_shade<4, MJ><<<cfg.shade_fam_blocks[4], shade_threads(4), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      if (cfg.family_mask & (1u << 5)) k_shade<5, MJ><<<cfg.shade_fam_blocks[5], shade_threads(5), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      if (cfg.family_mask & (1u << 6)) k_shade<6, MJ><<<cfg.shade_fam_blocks[6], shade_threads(6), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
+      k_shade<PT_FAM_MISC, MJ><<<cfg.shade_fam_blocks[PT_FAM_MISC], shade_threads(PT_FAM_MISC), 0, next_stream()>>>(S, J, T, Q, qsel, b, g0, LN);
       for (int u = 0; u < used; ++u) {
         cudaEventRecord(ss->join[u], ss->aux[u]);
         cudaStreamWaitEvent(st, ss->join[u], 0);
@@ -1090,7 +1163,7 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
       P.count(STAGE_SHADE, 1 + __builtin_popcount(cfg.family_mask & 0x7fu));
     } else {
       P.begin(STAGE_SHADE, st);
-      k_shade<-1, MJ><<<cfg.shade_fam_blocks[PT_FAM_MISC + 1], 128, 0, st>>>(S, J, T, Q, qsel, b, g0);
+      k_shade<-1, MJ><<<cfg.shade_fam_blocks[PT_FAM_MISC + 1], 128, 0, st>>>(S, J, T, Q, qsel, b, g0, LN);
       P.end(st);
       P.count(STAGE_SHADE, 1);
     }
