@@ -1568,6 +1568,13 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
                                     j == 0 ? k.width0 : j == 1 ? k.width1 : 0.f);
     }
     V.curves = up(cv);
+    if (device) {
+      void *seg = nullptr;
+      cuda_check(cudaMalloc(&seg, sizeof(float4) * 2 * PT_CURVE_SEGMENTS * n_curves), "cudaMalloc(curves)");
+      S->owned.push_back(seg);
+      V.curve_segments = static_cast<float4 *>(seg);
+      launch_curve_segments(V.curves, n_curves, static_cast<float4 *>(seg), st);
+    }
   }
   if (!motion.empty()) {
     V.motion = up(motion);

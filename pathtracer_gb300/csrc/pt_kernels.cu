@@ -379,6 +379,18 @@ void launch_owen_tables(uint32_t *tables, uint32_t n, cudaStream_t st) {
   k_owen_tables<<<grid_for(n, 256, 152 * 16), 256, 0, st>>>(tables, n);
 }
 
+// The curves' segments, one per thread (a scene upload).
+__global__ void k_curve_segments(const float4 *curves, int n, float4 *out) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n * PT_CURVE_SEGMENTS; i += gridDim.x * blockDim.x) {
+    const CurveSegment g = curve_segment(curves + 4 * (size_t)(i / PT_CURVE_SEGMENTS), i % PT_CURVE_SEGMENTS);
+    out[2 * (size_t)i] = make_float4(g.pa.x, g.pa.y, g.pa.z, g.radius);
+    out[2 * (size_t)i + 1] = make_float4(g.axis.x, g.axis.y, g.axis.z, g.len);
+  }
+}
+void launch_curve_segments(const float4 *curves, int n, float4 *out, cudaStream_t st) {
+  k_curve_segments<<<grid_for((long long)n * PT_CURVE_SEGMENTS, 128, 152 * 16), 128, 0, st>>>(curves, n, out);
+}
+
 // The traversal's nodes from the built ones, one per thread (a scene upload).
 __global__ void k_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = pack_node(nodes[i]);

@@ -140,6 +140,7 @@ struct KernelInfo {
 
 void upload_halton_tables(const HaltonTables &T, cudaStream_t st);
 void launch_owen_tables(uint32_t *tables, uint32_t n, cudaStream_t st);
+void launch_curve_segments(const float4 *curves, int n, float4 *out, cudaStream_t st);
 void launch_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out, cudaStream_t st);
 void launch_light_eval(const SceneView &S, int light, int n, const float *uv, const float *x, const float *pdf_dir,
                        float *point, float *normal, float *dir, float *le, float *pdf, cudaStream_t st);

@@ -21,6 +21,8 @@
 #define PT_STACK 48
 #endif
 #define PT_STACK_SHARED 16
+// Cylinders a curve is intersected as (primitives/curve.hpp).
+#define PT_CURVE_SEGMENTS 8
 
 namespace pt {
 
@@ -132,6 +134,7 @@ struct SceneView {
   const float4 *prim_uv;   // per primitive texture-coordinate records (null: no textures)
   int32_t n_textures;
   const float4 *curves;    // per curve: (cp0, width0), (cp1, width1), (cp2, 0), (cp3, 0)
+  const float4 *curve_segments;  // per curve and segment: (start, radius), (axis, length)
 };
 
 // Child references of a BVH4 node entering a moving object's subtree carry

@@ -92,6 +92,13 @@ __device__ __forceinline__ bool hit_sphere(const Item &it, V3 o, V3 dn, float tm
   return true;
 }
 
+// 32 bytes with one load.
+__device__ __forceinline__ void ld32b(const void *p, uint32_t *v) {
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+      : "l"(p));
+}
+
 // Cubic Bezier point and derivative (primitives/bezier.hpp:10-36).
 // Bezier point with every operation separately rounded (never fused), in
 // bezier.hpp:10-18's order, so that curve hits round like the reference's.
@@ -114,13 +121,38 @@ __device__ __forceinline__ V3 bezier_tangent(const float4 *cp, float u) {
   return d0 * (u1 * u1) + d1 * (2.0f * u * u1) + d2 * (u * u);
 }
 
-// Curve::intersect (primitives/curve.hpp:48-129): the Bezier split into 8
-// segments, each an infinite cylinder of the segment's mean radius cut at its
-// ends; roots from gl::solveQuadratic (utility.hpp:112-124).  Returns the
-// segment in u and the position along it in v (fraction of its length).
-__device__ __forceinline__ bool hit_curve(const float4 *cp, V3 o, V3 d, float tmin, float tmax, float &t_out,
+// Segment i of a curve, an infinite cylinder cut at its ends
+// (primitives/curve.hpp:48-103): start point and radius (the mean of the
+// linearly interpolated width at the ends), axis and length.
+struct CurveSegment {
+  V3 pa;
+  float radius;
+  V3 axis;
+  float len;
+};
+__device__ __forceinline__ CurveSegment curve_segment(const float4 *cp, int i) {
+  const int N = PT_CURVE_SEGMENTS;
+  const float u0 = float(i) / N, u1 = float(i + 1) / N;
+  const V3 pa = bezier_point(cp, u0), pb = bezier_point(cp, u1);
+  const float w0 = __ldg(cp).w, w1 = __ldg(cp + 1).w;
+  const float r0 = xadd(w0, xmul(xsub(w1, w0), u0)), r1 = xadd(w0, xmul(xsub(w1, w0), u1));
+  const V3 ab = xsubv(pb, pa);
+  CurveSegment g;
+  g.pa = pa;
+  g.radius = xmul(0.5f, xadd(r0, r1));
+  g.len = xsqrt(xdot(ab, ab));
+  g.axis = v3(xdiv(ab.x, g.len), xdiv(ab.y, g.len), xdiv(ab.z, g.len));
+  return g;
+}
+
+// Curve::intersect (primitives/curve.hpp:48-129) over the curve's segments
+// (8 x 32 B); roots from gl::solveQuadratic (utility.hpp:112-124).  Returns
+// the segment in u and the position along it in v (fraction of its length).
+// The segments are tabulated at upload by curve_segment: computing them in the
+// test took two thirds of it (two Bezier points, a root and three divisions
+// per segment and ray); hair on curves, 0.96 M paths: trace 5.9 -> 4.4 ms.
+__device__ __forceinline__ bool hit_curve(const float4 *seg, V3 o, V3 d, float tmin, float tmax, float &t_out,
                                           float &u_out, float &v_out) {
-  const int N = 8;
   float best = tmax;
   bool found = false;
   // Exact (never fused) arithmetic throughout: the cylinder quadratic is
@@ -129,18 +161,12 @@ __device__ __forceinline__ bool hit_curve(const float4 *cp, V3 o, V3 d, float tm
   auto axpy = [](V3 a, float k, V3 b) {  // a - k b
     return v3(xsub(a.x, xmul(k, b.x)), xsub(a.y, xmul(k, b.y)), xsub(a.z, xmul(k, b.z)));
   };
-  // the end points are recomputed per segment (as the reference does) and
-  // the widths reloaded, which keeps fewer values live in the traversal loop
 #pragma unroll 1
-  for (int i = 0; i < N; ++i) {
-    const float u0 = float(i) / N, u1 = float(i + 1) / N;
-    const V3 pa = bezier_point(cp, u0), pb = bezier_point(cp, u1);
-    const float w0 = __ldg(cp).w, w1 = __ldg(cp + 1).w;
-    const float r0 = xadd(w0, xmul(xsub(w1, w0), u0)), r1 = xadd(w0, xmul(xsub(w1, w0), u1));
-    const float radius = xmul(0.5f, xadd(r0, r1));
-    const V3 ab = xsubv(pb, pa);
-    const float seg_len = xsqrt(xdot(ab, ab));
-    const V3 axis = v3(xdiv(ab.x, seg_len), xdiv(ab.y, seg_len), xdiv(ab.z, seg_len));
+  for (int i = 0; i < PT_CURVE_SEGMENTS; ++i) {
+    uint32_t w[8];
+    ld32b(seg + 2 * i, w);
+    const V3 pa = v3(u2f(w[0]), u2f(w[1]), u2f(w[2])), axis = v3(u2f(w[4]), u2f(w[5]), u2f(w[6]));
+    const float radius = u2f(w[3]), seg_len = u2f(w[7]);
     const V3 d_perp = axpy(d, xdot(d, axis), axis);
     const V3 delta = xsubv(o, pa);
     const V3 o_perp = axpy(delta, xdot(delta, axis), axis);
@@ -208,7 +234,7 @@ __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V
   if (type == ITEM_TRI) {
     h = hit_triangle(it, o, d, tmin, tmax, t, u, v);
   } else if (CURVES && type == ITEM_CURVE) {
-    h = hit_curve(S.curves + 4 * (size_t)f2u(it.a[0]), o, d, tmin, tmax, t, u, v);
+    h = hit_curve(S.curve_segments + 2 * PT_CURVE_SEGMENTS * (size_t)f2u(it.a[0]), o, d, tmin, tmax, t, u, v);
   } else if (type == ITEM_CURVE) {
     h = false;
   } else {
@@ -328,13 +354,6 @@ __device__ __forceinline__ void fma2(uint32_t u0, uint32_t u1, uint64_t a, uint6
       : "=f"(t0), "=f"(t1)
       : "r"(u0), "r"(u1), "l"(a), "l"(c));
 }
-// 32 bytes of a node with one load.
-__device__ __forceinline__ void ld32b(const void *p, uint32_t *v) {
-  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-      : "l"(p));
-}
-
 // Visits node R.ref: afterwards R.ref is the next reference (SORTED: the
 // nearest hit child, the others pushed far first; else the first hit child in
 // node order), or the top of the stack when no child is hit.  Returns false
