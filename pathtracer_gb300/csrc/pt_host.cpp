@@ -170,12 +170,33 @@ MatRec derive_material(const pt_material_desc &m) {
   return r;
 }
 
+// A vector that leaves its new elements uninitialised: arrays whose every
+// element a parallel_for writes (zeroing them first would touch each page on
+// one thread).
+template <class T>
+struct NoInit : std::allocator<T> {
+  template <class U>
+  struct rebind {
+    using other = NoInit<U>;
+  };
+  template <class U>
+  void construct(U *p) {
+    ::new (static_cast<void *>(p)) U;
+  }
+  template <class U, class... A>
+  void construct(U *p, A &&...a) {
+    ::new (static_cast<void *>(p)) U(std::forward<A>(a)...);
+  }
+};
+template <class T>
+using RawVec = std::vector<T, NoInit<T>>;
+
 // Runs f(i) for i in [0, n) on up to `threads` host threads (0: all
-// hardware threads), in contiguous chunks; f must touch disjoint state per i.
+// hardware threads), in contiguous chunks of at least `grain`; f must touch
+// disjoint state per i.
 template <class F>
-static void parallel_for(size_t n, int threads, F f) {
+static void parallel_for(size_t n, int threads, F f, size_t grain = 1 << 15) {
   unsigned hw = threads > 0 ? (unsigned)threads : std::max(1u, std::thread::hardware_concurrency());
-  const size_t grain = 1 << 15;
   const unsigned nt = (unsigned)std::min<size_t>(hw, (n + grain - 1) / grain);
   if (nt <= 1) {
     for (size_t i = 0; i < n; ++i) f(i);
@@ -889,8 +910,198 @@ static void collapse(const Builder &B, int bn, Bvh4Out &out, int depth, int me, 
   }
 }
 
-template <class T>
-static T *dupload(const std::vector<T> &v, std::vector<void *> &owned, cudaStream_t st) {
+// ------------------------------------------------- the any-hit rays' top
+// Whether anything occludes a ray does not depend on the tree, so any-hit rays
+// enter through a top of their own: the largest nodes of the BVH4 are opened
+// into at most `max_units` subtrees and leaves, which an exact surface-area
+// sweep groups anew (the reference's object level halves the insertion order,
+// its meshes are split at the median).  Everything below is shared.  Returns
+// the new nodes, the root first (child indices of new nodes continue behind
+// the `out.nodes`), or none when the sweep's nodes are not smaller in all or a
+// ray's stack would not hold the deeper tree.  Shadow rays of the Cornell box
+// 6.42 -> 5.72 ms, hair on curves (paired launches) 4.42 -> 3.58, material
+// divergence 24.5 -> 24.1; one mesh alone does not change.  128 / 512 / 2048
+// units: Cornell 5.73 / 5.72 / 5.59, hair 4.05 / 3.58 / 3.57 (202 objects); the
+// sweep takes 0.3 ms of an upload at 256.
+// Subtrees and leaves an any-hit top groups.
+#define PT_TOP_UNITS 256
+struct TopUnit {
+  Box box;
+  int32_t child, count;
+  int depth;  // levels of nodes above it in the BVH4
+};
+struct TopNode {
+  Box box;
+  int left = -1, right = -1, unit = -1;
+};
+// The sweep over units [lo, hi) of ord[axis], the units in centroid order per
+// axis: each split keeps the three orders (a stable partition), so they are
+// sorted once.
+static int top_sweep(const std::vector<TopUnit> &units, std::vector<int> (&ord)[3], std::vector<float> &right,
+                     std::vector<char> &goes_left, std::vector<int> &tmp, int lo, int hi, std::vector<TopNode> &out) {
+  const int me = (int)out.size();
+  out.emplace_back();
+  if (hi - lo == 1) {
+    out[me].unit = ord[0][lo];
+    out[me].box = units[ord[0][lo]].box;
+    return me;
+  }
+  float best = INFINITY;
+  int split = lo + (hi - lo) / 2, axis = 0;
+  auto weight = [&](int u) { return units[u].count > 0 ? 1.f : 3.f; };
+  for (int a = 0; a < 3; ++a) {
+    const std::vector<int> &o = ord[a];
+    Box b = units[o[hi - 1]].box;
+    float w = 0.f;
+    for (int k = hi - 1; k > lo; --k) {
+      b = box_merge(b, units[o[k]].box);
+      w += weight(o[k]);
+      right[k] = box_area(b) * w;
+    }
+    if (a == 0) out[me].box = box_merge(b, units[o[lo]].box);
+    b = units[o[lo]].box;
+    w = 0.f;
+    for (int k = lo + 1; k < hi; ++k) {
+      b = box_merge(b, units[o[k - 1]].box);
+      w += weight(o[k - 1]);
+      const float cost = box_area(b) * w + right[k];
+      if (cost < best) {
+        best = cost;
+        split = k;
+        axis = a;
+      }
+    }
+  }
+  for (int k = lo; k < hi; ++k) goes_left[ord[axis][k]] = k < split;
+  for (int a = 0; a < 3; ++a) {
+    if (a == axis) continue;
+    int l = lo, r = 0;
+    for (int k = lo; k < hi; ++k) {
+      const int u = ord[a][k];
+      if (goes_left[u]) ord[a][l++] = u;
+      else tmp[r++] = u;
+    }
+    std::copy(tmp.begin(), tmp.begin() + r, ord[a].begin() + l);
+  }
+  const int l = top_sweep(units, ord, right, goes_left, tmp, lo, split, out);
+  const int r = top_sweep(units, ord, right, goes_left, tmp, split, hi, out);
+  out[me].left = l;
+  out[me].right = r;
+  return me;
+}
+static std::vector<Bvh4Node> any_hit_top(const Bvh4Out &out, int max_units) {
+  std::vector<Bvh4Node> top;
+  std::vector<TopUnit> units;
+  std::vector<std::pair<float, int>> heap;  // (area, unit) of the nodes that may be opened
+  float area_before = 0.f;
+  auto open = [&](int node, int depth, int slot) {
+    const Bvh4Node &N = out.nodes[node];
+    for (int k = 0; k < 4; ++k) {
+      if (N.count[k] < 0) continue;
+      TopUnit u;
+      const float lo[3] = {N.lo_x[k], N.lo_y[k], N.lo_z[k]}, hi[3] = {N.hi_x[k], N.hi_y[k], N.hi_z[k]};
+      for (int a = 0; a < 3; ++a) {
+        u.box.lo[a] = lo[a];
+        u.box.hi[a] = hi[a];
+      }
+      u.child = N.child[k];
+      u.count = N.count[k];
+      u.depth = depth + 1;
+      if (slot < 0) {
+        slot = (int)units.size();
+        units.emplace_back();
+      }
+      units[slot] = u;
+      if (u.count == 0 && !(u.child & PT_INST_BIT)) {
+        heap.emplace_back(box_area(u.box), slot);
+        std::push_heap(heap.begin(), heap.end());
+      }
+      slot = -1;
+    }
+  };
+  open(0, 0, -1);
+  while (!heap.empty() && (int)units.size() + 3 <= max_units) {
+    std::pop_heap(heap.begin(), heap.end());
+    const auto [area, u] = heap.back();
+    heap.pop_back();
+    area_before += area;
+    open(units[u].child, units[u].depth, u);
+  }
+  if (area_before == 0.f) return top;  // one node: nothing to group
+  const int n = (int)units.size();
+  std::vector<int> ord[3], tmp(n);
+  std::vector<float> right(n), centre(n);
+  std::vector<char> goes_left(n);
+  for (int a = 0; a < 3; ++a) {
+    ord[a].resize(n);
+    for (int k = 0; k < n; ++k) {
+      ord[a][k] = k;
+      centre[k] = units[k].box.lo[a] + units[k].box.hi[a];
+    }
+    std::sort(ord[a].begin(), ord[a].end(),
+              [&](int x, int y) { return centre[x] != centre[y] ? centre[x] < centre[y] : x < y; });
+  }
+  std::vector<TopNode> bin;
+  bin.reserve(2 * n);
+  top_sweep(units, ord, right, goes_left, tmp, 0, n, bin);
+  const int base = (int)out.nodes.size();
+  float area_after = 0.f;
+  int levels = 0;
+  // collapsed as the whole tree is: the largest child is opened until there
+  // are four
+  struct Todo {
+    int bn, node, level;
+  };
+  std::vector<Todo> todo{{0, 0, 1}};
+  top.emplace_back();
+  while (!todo.empty()) {
+    const Todo t = todo.back();
+    todo.pop_back();
+    if (t.node > 0) area_after += box_area(bin[t.bn].box);
+    int ch[4] = {bin[t.bn].left, bin[t.bn].right, -1, -1}, nch = 2;
+    while (nch < 4) {
+      int best = -1;
+      for (int k = 0; k < nch; ++k)
+        if (bin[ch[k]].unit < 0 && (best < 0 || box_area(bin[ch[k]].box) > box_area(bin[ch[best]].box))) best = k;
+      if (best < 0) break;
+      const int x = ch[best];
+      ch[best] = bin[x].left;
+      ch[nch++] = bin[x].right;
+    }
+    Bvh4Node N;
+    for (int k = 0; k < 4; ++k) {
+      N.lo_x[k] = N.lo_y[k] = N.lo_z[k] = INFINITY;
+      N.hi_x[k] = N.hi_y[k] = N.hi_z[k] = -INFINITY;
+      N.child[k] = 0;
+      N.count[k] = -1;
+      if (k >= nch) continue;
+      const TopNode &c = bin[ch[k]];
+      N.lo_x[k] = c.box.lo[0];
+      N.lo_y[k] = c.box.lo[1];
+      N.lo_z[k] = c.box.lo[2];
+      N.hi_x[k] = c.box.hi[0];
+      N.hi_y[k] = c.box.hi[1];
+      N.hi_z[k] = c.box.hi[2];
+      if (c.unit >= 0) {
+        const TopUnit &u = units[c.unit];
+        N.child[k] = u.child;
+        N.count[k] = u.count;
+        levels = std::max(levels, t.level + (u.count > 0 ? 0 : out.max_depth - u.depth));
+      } else {
+        N.child[k] = base + (int)top.size();
+        N.count[k] = 0;
+        todo.push_back({ch[k], (int)top.size(), t.level + 1});
+        top.emplace_back();
+      }
+    }
+    top[t.node] = N;
+  }
+  if (!(area_after < area_before) || 3 * levels + 2 > PT_STACK) top.clear();
+  return top;
+}
+
+template <class T, class A>
+static T *dupload(const std::vector<T, A> &v, std::vector<void *> &owned, cudaStream_t st) {
   if (v.empty()) return nullptr;
   void *p = nullptr;
   cuda_check(cudaMalloc(&p, sizeof(T) * v.size()), "cudaMalloc(scene)");
@@ -1181,15 +1392,13 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
     fail(PT_ERR_TOO_LARGE, "BVH deeper than the traversal stack (" + std::to_string(out.max_depth) + ")");
 
   // leaf items and shading records
-  std::vector<Item> items(out.leaf_order.size());
-  std::vector<PrimShade> shade(n_prims);
+  RawVec<Item> items(out.leaf_order.size());
+  RawVec<PrimShade> shade(n_prims);
   std::vector<int> prim_item(n_prims, -1);
-  std::vector<int> prim_mesh(B.n_tris), prim_tri(B.n_tris);
-  for (int m = 0; m < d->n_meshes; ++m)
-    for (int t = 0; t < d->meshes[m].n_triangles; ++t) {
-      prim_mesh[B.tri_base[m] + t] = m;
-      prim_tri[B.tri_base[m] + t] = t;
-    }
+  // mesh of a triangle: the last one that begins at or before it
+  auto mesh_of = [&](int prim) {
+    return (int)(std::upper_bound(B.tri_base.begin(), B.tri_base.end(), prim) - B.tri_base.begin()) - 1;
+  };
   parallel_for(out.leaf_order.size(), threads, [&](size_t k) {
     const int prim = out.leaf_order[k];
     Item &it = items[k];
@@ -1200,8 +1409,8 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
     it.c[3] = u2f((uint32_t)(out.leaf_world[k] ? prim_motion[prim] : 0));
     prim_item[prim] = (int)k;
     if (prim < B.n_tris) {
-      const pt_mesh_desc &m = d->meshes[prim_mesh[prim]];
-      const int t = prim_tri[prim];
+      const int mi = mesh_of(prim), t = prim - B.tri_base[mi];
+      const pt_mesh_desc &m = d->meshes[mi];
       const float *p0 = m.positions + 3 * m.indices[3 * t];
       const float *p1 = m.positions + 3 * m.indices[3 * t + 1];
       const float *p2 = m.positions + 3 * m.indices[3 * t + 2];
@@ -1240,8 +1449,8 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
     ps.light = -1;
     ps.flags = (prim_motion[prim] << 8) | prim_face[prim];
     if (prim < B.n_tris) {
-      const pt_mesh_desc &m = d->meshes[prim_mesh[prim]];
-      const int t = prim_tri[prim];
+      const int mi = mesh_of(prim), t = prim - B.tri_base[mi];
+      const pt_mesh_desc &m = d->meshes[mi];
       ps.material = m.material;
       ps.flags |= ITEM_TRI << 2;
       {
@@ -1286,10 +1495,13 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   // materials
   std::vector<MatRec> mats;
   for (int i = 0; i < d->n_materials; ++i) mats.push_back(derive_material(d->materials[i]));
-  for (int prim = 0; prim < n_prims; ++prim) {
-    const int t = mats[shade[prim].material].type;
+  auto uses = [&](int material) {
+    const int t = mats[material].type;
     if (t < PT_MAT_DIFFUSE_EMITTER) S->family_mask |= 1u << t;
-  }
+  };
+  for (int m = 0; m < d->n_meshes; ++m)
+    if (d->meshes[m].n_triangles > 0) uses(d->meshes[m].material);
+  for (int prim = B.n_tris; prim < n_prims; ++prim) uses(shade[prim].material);
 
   // textures (ColorVariant): the table, an image texel pool, and per
   // primitive texture-coordinate records when a material uses one
@@ -1331,7 +1543,7 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
     for (int prim = 0; prim < n_prims; ++prim) {
       float4 &a = prim_uv[2 * prim], &b = prim_uv[2 * prim + 1];
       if (prim < B.n_tris) {
-        const int mi = prim_mesh[prim], t = prim_tri[prim];
+        const int mi = mesh_of(prim), t = prim - B.tri_base[mi];
         const pt_mesh_desc &m = d->meshes[mi];
         if (m.uvs && m.n_uvs > 0) {
           // MeshBVHNode::hitTriangle's uv interpolation (meshBVH.cpp:134-138);
@@ -1430,32 +1642,40 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   }
 
   // environment map + luminance alias table
-  std::vector<float4> tex;
-  std::vector<float> aprob, apdf;
-  std::vector<int32_t> aidx;
+  RawVec<float4> tex;
+  RawVec<float> aprob, apdf;
+  RawVec<int32_t> aidx;
   if (d->env) {
     const pt_env_desc &e = *d->env;
     if (!e.texels || e.width < 2 || e.height < 2) fail(PT_ERR_INVALID, "environment map smaller than 2x2");
     const int W = e.width, H = e.height, N = W * H;
+    const size_t few = 1 << 17;  // light loops: starting a thread costs ~50 us
     tex.resize(N);
-    for (int i = 0; i < N; ++i) tex[i] = make_float4(e.texels[3 * i], e.texels[3 * i + 1], e.texels[3 * i + 2], 0.f);
+    parallel_for((size_t)N, threads, [&](size_t i) {
+      tex[i] = make_float4(e.texels[3 * i], e.texels[3 * i + 1], e.texels[3 * i + 2], 0.f);
+    }, few);
     // cell (x, y) covers u in [x/W, (x+1)/W): weight = mean luminance of the
     // texels the bilinear lookup blends there, times sin(theta), plus a floor
-    std::vector<double> w(N);
-    double sum = 0.0;
-    for (int y = 0; y < H; ++y)
-      for (int x = 0; x < W; ++x) {
-        double l = 0.0;
-        for (int dy = 0; dy < 2; ++dy)
-          for (int dx = 0; dx < 2; ++dx) {
-            int xx = std::min(x + dx, W - 1), yy = std::min(y + dy, H - 1);
-            const float4 &t = tex[yy * W + xx];
-            l += 0.2126 * t.x + 0.7152 * t.y + 0.0722 * t.z;
+    RawVec<double> w(N);
+    parallel_for(
+        (size_t)H, threads,
+        [&](size_t row) {
+          const int y = (int)row;
+          const double st = std::sin(PT_PI * (y + 0.5) / H);
+          for (int x = 0; x < W; ++x) {
+            double l = 0.0;
+            for (int dy = 0; dy < 2; ++dy)
+              for (int dx = 0; dx < 2; ++dx) {
+                int xx = std::min(x + dx, W - 1), yy = std::min(y + dy, H - 1);
+                const float4 &t = tex[yy * W + xx];
+                l += 0.2126 * t.x + 0.7152 * t.y + 0.0722 * t.z;
+              }
+            w[y * W + x] = std::max(0.0, l * 0.25) * st;
           }
-        double st = std::sin(PT_PI * (y + 0.5) / H);
-        w[y * W + x] = std::max(0.0, l * 0.25) * st;
-        sum += w[y * W + x];
-      }
+        },
+        std::max<size_t>(1, few / (size_t)W));
+    double sum = 0.0;  // in index order
+    for (int i = 0; i < N; ++i) sum += w[i];
     double floor_w = (sum > 0 ? sum / N : 1.0) * 1e-3;
     sum = 0.0;
     for (int y = 0; y < H; ++y) {
@@ -1466,17 +1686,20 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
       }
     }
     apdf.resize(N);
-    for (int i = 0; i < N; ++i) apdf[i] = (float)(w[i] / sum);
     // Vose's alias method
-    aprob.assign(N, 1.f);
+    aprob.resize(N);
     aidx.resize(N);
-    std::vector<double> sc(N);
-    std::vector<int> small, large;
-    for (int i = 0; i < N; ++i) {
+    RawVec<double> sc(N);
+    parallel_for((size_t)N, threads, [&](size_t i) {
+      apdf[i] = (float)(w[i] / sum);
+      aprob[i] = 1.f;
       sc[i] = w[i] / sum * N;
-      aidx[i] = i;
-      (sc[i] < 1.0 ? small : large).push_back(i);
-    }
+      aidx[i] = (int32_t)i;
+    }, few);
+    std::vector<int> small, large;
+    small.reserve(N);
+    large.reserve(N);
+    for (int i = 0; i < N; ++i) (sc[i] < 1.0 ? small : large).push_back(i);
     while (!small.empty() && !large.empty()) {
       int s = small.back(); small.pop_back();
       int l = large.back(); large.pop_back();
@@ -1515,14 +1738,18 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
       for (void *p : v) cudaFree(p);
     }
   } freed{staged};
+  int any_root = 0;
   if (device) {
     // packed on the device; the host tree and its hash keep the float boxes
-    const Bvh4Node *wide = dupload(out.nodes, staged, st);
+    const std::vector<Bvh4Node> top = any_hit_top(out, PT_TOP_UNITS);
+    any_root = top.empty() ? 0 : (int)out.nodes.size();
+    const Bvh4Node *wide = dupload(out.nodes, staged, st), *wide_top = dupload(top, staged, st);
     void *packed = nullptr;
-    cuda_check(cudaMalloc(&packed, sizeof(PackedNode) * out.nodes.size()), "cudaMalloc(nodes)");
+    cuda_check(cudaMalloc(&packed, sizeof(PackedNode) * (out.nodes.size() + top.size())), "cudaMalloc(nodes)");
     S->owned.push_back(packed);
     S->nodes = static_cast<PackedNode *>(packed);
     launch_pack_nodes(wide, (int)out.nodes.size(), S->nodes, st);
+    if (!top.empty()) launch_pack_nodes(wide_top, (int)top.size(), S->nodes + out.nodes.size(), st);
   }
   S->items = up(items);
   S->shade = up(shade);
@@ -1538,6 +1765,7 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   V.n_lights = (int)lights.size();
   S->host_lights = lights;
   V.n_nodes = (int)out.nodes.size();
+  V.any_root = any_root;
   V.n_prims = n_prims;
   V.trav_cap = trav_cap > 0 ? trav_cap : PT_TRAVERSAL_CAP;
   for (int c = 0; c < 3; ++c) V.bg[c] = d->bg_color[c];
@@ -1650,9 +1878,9 @@ Context::Context(int dev) : device(dev) {
   cfg.pair_from_bounce = 0;
   const char *pfb = std::getenv("PT_PAIR_FROM_BOUNCE");
   if (pfb) cfg.pair_from_bounce = std::max(0, std::atoi(pfb));
-  cuda_check(cudaMalloc(&d_err, 2 * sizeof(int)), "cudaMalloc(err)");
+  cuda_check(cudaMalloc(&d_err, 3 * sizeof(int)), "cudaMalloc(err)");
   d_fetch = d_err + 1;
-  cuda_check(cudaMemsetAsync(d_err, 0, 2 * sizeof(int), stream), "memset err");
+  cuda_check(cudaMemsetAsync(d_err, 0, 3 * sizeof(int), stream), "memset err");
   cuda_check(cudaStreamSynchronize(stream), "context init");
 }
 
@@ -2374,7 +2602,7 @@ static int trace_common(void *ctx, int32_t scene_id, bool any, const float *rays
     uint8_t *docc = (uint8_t *)(buf + nn * 44);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
     if (any) cuda_check(cudaMemcpyAsync(dtm, tmaxs, nn * 4, cudaMemcpyHostToDevice, c->stream), "h2d tmax");
-    launch_trace_test(S->view, any, dr, dtm, n, tmin, tmax, dt, dp, duv, docc, c->d_fetch, c->d_err, c->stream);
+    launch_trace_test(S->view, any, dr, dtm, n, tmin, tmax, dt, dp, duv, docc, c->next_fetch(), c->d_err, c->stream);
     cuda_check(cudaGetLastError(), "trace launch");
     if (any) {
       cuda_check(cudaMemcpyAsync(occ, docc, nn, cudaMemcpyDeviceToHost, c->stream), "d2h");
@@ -2422,7 +2650,7 @@ int pt_intersect(void *ctx, int32_t scene_id, const float *rays, int32_t n, floa
     float *dn = (float *)(buf + nn * 44);
     uint8_t *df = (uint8_t *)(buf + nn * 56);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
-    launch_intersect(S->view, dr, n, tmin, tmax, dt, dp, dpos, dn, df, c->d_fetch, c->d_err, c->stream);
+    launch_intersect(S->view, dr, n, tmin, tmax, dt, dp, dpos, dn, df, c->next_fetch(), c->d_err, c->stream);
     cuda_check(cudaGetLastError(), "intersect launch");
     cuda_check(cudaMemcpyAsync(t, dt, nn * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
     cuda_check(cudaMemcpyAsync(prim, dp, nn * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");

@@ -136,7 +136,12 @@ struct Context {
   size_t scratch_cap = 0;
   uint32_t *d_owen = nullptr;  // first digits of the Owen-scrambled dimensions (11 MB, as long as the context)
   int *d_err = nullptr;    // device error flag
-  int *d_fetch = nullptr;  // fetch counter of the ray-query kernels (behind d_err)
+  int *d_fetch = nullptr;  // two fetch counters of the ray queries (behind d_err), in turn
+  int fetch_turn = 0;
+  FetchPair next_fetch() {
+    fetch_turn ^= 1;
+    return FetchPair{d_fetch + fetch_turn, d_fetch + (fetch_turn ^ 1)};
+  }
   Profiler prof;
   Batch batch;
   int batch_wave_cap = 1 << 22;  // paths per wave of each batched job

@@ -68,16 +68,23 @@ void launch_path_samples(const DeviceJob &J, long long first, int n, int dims, i
   k_path_samples<<<grid_for(n, 128, 152 * 8), 128, 0, st>>>(J, first, n, dims, bounces, LN, pix, dv, lo);
 }
 
-// The batch ray queries: closest hits or occlusion of n given rays, *fetch = 0
-// at the start.
+// Blocks of a query: the warps of the whole chip, down to 4 rays per warp (a
+// warp of few rays ends sooner: its rays do not wait for each other's turns).
+static int query_grid(int n) { return grid_for(n, 16, 152 * 7); }
+
+// The batch ray queries: closest hits or occlusion of n given rays.  fetch.now
+// is 0 at the start; the kernel clears fetch.next for the next query (queries of
+// a context take turns, which saves clearing it by a memset: 2 of ~110 us for
+// 2500 rays).
 template <bool ANY, bool CURVES, bool MOTION>
 __global__ void __launch_bounds__(128) k_trace_test(SceneView S, const float *rays, const float *tmaxs, int n,
                                                     float tmin, float tmax, float *t_out, int *prim_out, float *uv_out,
-                                                    uint8_t *occ, int *fetch, int *err) {
+                                                    uint8_t *occ, FetchPair fetch, int *err) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
+  if (blockIdx.x == 0 && threadIdx.x == 0) *fetch.next = 0;
   int i = 0;
   trace_rays<ANY ? TRACE_ANY : TRACE_CLOSEST, CURVES, MOTION>(
-      S, n, fetch, ANY ? PT_FETCH_IDLE_SHADOW : PT_FETCH_IDLE, err, smem,
+      S, n, fetch.now, ANY ? PT_FETCH_IDLE_SHADOW : PT_FETCH_IDLE, err, smem,
       [&](int r, V3 &o, V3 &d, float &t0, float &t1, float &, bool &) {
         i = r;
         const float *p = rays + 6 * (size_t)r;
@@ -105,11 +112,12 @@ __global__ void __launch_bounds__(128) k_trace_test(SceneView S, const float *ra
 // toggled) -- what surface_at gives the shade stage.
 __global__ void __launch_bounds__(128) k_intersect(SceneView S, const float *rays, int n, float tmin, float tmax,
                                                    float *t_out, int *prim_out, float *pos, float *nrm,
-                                                   uint8_t *front, int *fetch, int *err) {
+                                                   uint8_t *front, FetchPair fetch, int *err) {
   extern __shared__ __align__(16) char smem[];  // trace_smem
+  if (blockIdx.x == 0 && threadIdx.x == 0) *fetch.next = 0;
   int i = 0;
   trace_rays<TRACE_CLOSEST, true, true>(
-      S, n, fetch, PT_FETCH_IDLE, err, smem,
+      S, n, fetch.now, PT_FETCH_IDLE, err, smem,
       [&](int r, V3 &o, V3 &d, float &t0, float &t1, float &, bool &) {
         i = r;
         const float *p = rays + 6 * (size_t)r;
@@ -138,9 +146,8 @@ __global__ void __launch_bounds__(128) k_intersect(SceneView S, const float *ray
 }
 
 void launch_intersect(const SceneView &S, const float *rays, int n, float tmin, float tmax, float *t, int *prim,
-                      float *pos, float *nrm, uint8_t *front, int *fetch, int *err, cudaStream_t st) {
-  cudaMemsetAsync(fetch, 0, sizeof(int), st);
-  k_intersect<<<grid_for(n, 128, 152 * 7), 128, trace_smem(128), st>>>(S, rays, n, tmin, tmax, t, prim, pos, nrm,
+                      float *pos, float *nrm, uint8_t *front, FetchPair fetch, int *err, cudaStream_t st) {
+  k_intersect<<<query_grid(n), 128, trace_smem(128), st>>>(S, rays, n, tmin, tmax, t, prim, pos, nrm,
                                                                          front, fetch, err);
 }
 
@@ -414,16 +421,15 @@ void launch_sampler_eval(int strategy, const uint16_t *perm, uint32_t first, int
 }
 
 void launch_trace_test(const SceneView &S, bool any, const float *rays, const float *tmaxs, int n,
-                       float tmin, float tmax, float *t, int *prim, float *uv, uint8_t *occ, int *fetch, int *err,
+                       float tmin, float tmax, float *t, int *prim, float *uv, uint8_t *occ, FetchPair fetch, int *err,
                        cudaStream_t st) {
-  const int g = grid_for(n, 128, 152 * 7);
-  cudaMemsetAsync(fetch, 0, sizeof(int), st);
+  const int g = query_grid(n);
 #define PT_RUN(C, M)                                                                                             \
   if (any)                                                                                                       \
-    k_trace_test<true, C, M><<<g, 128, trace_smem(128, true), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, \
+    k_trace_test<true, C, M><<<g, 128, trace_smem(128, true, M), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, \
                                                                        occ, fetch, err);                         \
   else                                                                                                           \
-    k_trace_test<false, C, M><<<g, 128, trace_smem(128), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, \
+    k_trace_test<false, C, M><<<g, 128, trace_smem(128, false, M), st>>>(S, rays, tmaxs, n, tmin, tmax, t, prim, uv, occ, \
                                                                   fetch, err)
   if (S.curves) {
     PT_RUN(true, true);
@@ -471,7 +477,7 @@ void launch_sort(const SceneView &S, const Queues &Q, int qsel, const LaunchCfg 
 }
 
 void launch_shadow(const SceneView &S, const Queues &Q, int LN, const LaunchCfg &cfg, cudaStream_t st) {
-#define PT_RUN(C, M) k_trace_shadow<C, M><<<cfg.trace_blocks, 128, trace_smem(128, true), st>>>(S, Q)
+#define PT_RUN(C, M) k_trace_shadow<C, M><<<cfg.trace_blocks, 128, trace_smem(128, true, M), st>>>(S, Q)
   PT_BY_SCENE(S, PT_RUN);
 #undef PT_RUN
   k_shadow_resolve<<<cfg.max_blocks_simple, 256, 0, st>>>(Q, LN);

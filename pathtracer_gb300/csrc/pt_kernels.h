@@ -132,6 +132,11 @@ struct Profiler {
   }
 };
 
+// Fetch counters of the ray queries: this one's (0) and the next one's.
+struct FetchPair {
+  int *now, *next;
+};
+
 struct KernelInfo {
   int trace_regs, shade_regs;
   int trace_blocks_per_sm, shade_blocks_per_sm, shadow_blocks_per_sm;
@@ -145,14 +150,14 @@ void launch_pack_nodes(const Bvh4Node *nodes, int n, PackedNode *out, cudaStream
 void launch_light_eval(const SceneView &S, int light, int n, const float *uv, const float *x, const float *pdf_dir,
                        float *point, float *normal, float *dir, float *le, float *pdf, cudaStream_t st);
 void launch_intersect(const SceneView &S, const float *rays, int n, float tmin, float tmax, float *t, int *prim,
-                      float *pos, float *nrm, uint8_t *front, int *fetch, int *err, cudaStream_t st);
+                      float *pos, float *nrm, uint8_t *front, FetchPair fetch, int *err, cudaStream_t st);
 void launch_path_samples(const DeviceJob &J, long long first, int n, int dims, int bounces, float *pix, float *dv,
                          float *lo, cudaStream_t st);
 void launch_sampler_eval(int strategy, const uint16_t *perm, uint32_t first, int n, int dims,
                          float *out, cudaStream_t st);
 void launch_trace_test(const SceneView &S, bool any, const float *rays, const float *tmaxs, int n,
                        float tmin, float tmax, float *t, int *prim, float *uv, uint8_t *occ,
-                       int *fetch, int *err, cudaStream_t st);
+                       FetchPair fetch, int *err, cudaStream_t st);
 void launch_bsdf_eval(const MatRec *m, int n, const float *wo, const float *wi, const float *nrm,
                       const uint8_t *front, float *f, float *pdf, cudaStream_t st);
 void launch_bsdf_sample(const MatRec *m, int n, const float *wo, const float *nrm,

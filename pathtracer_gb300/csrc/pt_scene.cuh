@@ -119,6 +119,7 @@ struct SceneView {
   const LightRec *lights;
   int32_t n_lights;
   int32_t n_nodes;
+  int32_t any_root;  // node any-hit rays start from (closest hits: node 0)
   int32_t n_prims;
   EnvMap env;
   float bg[3];

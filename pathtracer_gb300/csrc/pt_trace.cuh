@@ -296,8 +296,8 @@ enum TraceMode { TRACE_CLOSEST = 0, TRACE_ANY = 1, TRACE_MIXED = 2 };
 // Dynamic shared memory of a traversal block: the first PT_STACK_SHARED
 // entries of every thread's stack, the warps' records and the rays' world
 // origins (kernels for moving objects).
-inline size_t trace_smem(int threads, bool any_only = false) {
-  const size_t per = PT_STACK_SHARED * sizeof(int32_t) + 3 * sizeof(float);
+inline size_t trace_smem(int threads, bool any_only = false, bool motion = true) {
+  const size_t per = PT_STACK_SHARED * sizeof(int32_t) + (motion ? 3 * sizeof(float) : 0);
   return per * threads + (threads / 32) * (sizeof(WarpRays) + (any_only ? 0 : sizeof(WarpHits)));
 }
 
@@ -567,7 +567,8 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           }
           R.inv = v3(slab_inv(d.x), slab_inv(d.y), slab_inv(d.z));
           R.oi = v3(-o.x * R.inv.x, -o.y * R.inv.y, -o.z * R.inv.z);
-          R.ref = 0;  // node 0 is the root (the host always emits at least one node)
+          // the host always emits at least one node
+          R.ref = any ? S.any_root : 0;
           R.sp = 0;
           iters = 0;
           active = true;

@@ -1117,12 +1117,12 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
     if (pair) {
       // this bounce's closest rays with the previous bounce's shadow rays
 #define PT_RUN(C, M) \
-  k_trace_pair<MJ, C, M><<<cfg.trace_blocks, 128, trace_smem(128), st>>>(S, J, T, Q, qsel, b, g0)
+  k_trace_pair<MJ, C, M><<<cfg.trace_blocks, 128, trace_smem(128, false, M), st>>>(S, J, T, Q, qsel, b, g0)
       PT_BY_SCENE(S, PT_RUN);
 #undef PT_RUN
     } else {
 #define PT_RUN(C, M) \
-  k_trace_closest<MJ, C, M><<<cfg.trace_blocks, 128, trace_smem(128), st>>>(S, J, T, Q, qsel, b, g0)
+  k_trace_closest<MJ, C, M><<<cfg.trace_blocks, 128, trace_smem(128, false, M), st>>>(S, J, T, Q, qsel, b, g0)
       PT_BY_SCENE(S, PT_RUN);
 #undef PT_RUN
     }
