@@ -409,13 +409,13 @@ void render_batch(Context *c, const pt_job_desc *jobs, int n, float **films, pt_
       if (!films[k]) continue;
       const pt_job_desc &j = jobs[k];
       const size_t nf = (size_t)j.width * j.height * 3;
-      cuda_check(cudaMemcpy(films[k], slot.films + G.film_off[m], nf * sizeof(float), cudaMemcpyDeviceToHost),
-                 "film d2h");
+      float *df = slot.films + G.film_off[m];
       const int e = j.spp_end ? j.spp_end : j.spp_x * j.spp_y;
-      const float inv = 1.f / (float)(e - j.spp_begin);
-      for (size_t i = 0; i < nf; ++i) films[k][i] *= inv;
+      launch_film_scale(df, 1.f / (float)(e - j.spp_begin), (long long)nf, c->stream);
+      cuda_check(cudaMemcpyAsync(films[k], df, nf * sizeof(float), cudaMemcpyDeviceToHost, c->stream), "film d2h");
     }
   }
+  cuda_check(cudaStreamSynchronize(c->stream), "batch films");
   tot.ms = ms;
   tot.algorithmic_bytes = 192ull * tot.segments + 88ull * tot.shadow_rays + 24ull * tot.paths;
   if (stats) *stats = tot;

@@ -2411,6 +2411,9 @@ int pt_render(void *ctx, const pt_job_desc *job, float *film_rgb, pt_stats *stat
     float *df = c->film_buffer(nf);
     cuda_check(cudaMemsetAsync(df, 0, nf * sizeof(float), c->stream), "memset film");
     c->render_device(*job, df, stats, false);
+    // the mean, on the device (a 1080p film took the host 2 ms)
+    const int e = job->spp_end ? job->spp_end : job->spp_x * job->spp_y;
+    launch_film_scale(df, 1.f / (float)(e - job->spp_begin), (long long)nf, c->stream);
     cuda_check(cudaMemcpyAsync(film_rgb, df, nf * sizeof(float), cudaMemcpyDeviceToHost, c->stream), "film d2h");
     cuda_check(cudaStreamSynchronize(c->stream), "render");
     int herr = 0;
@@ -2419,9 +2422,6 @@ int pt_render(void *ctx, const pt_job_desc *job, float *film_rgb, pt_stats *stat
       cudaMemset(c->d_err, 0, sizeof(int));
       fail(PT_ERR_DEVICE, "device traversal error flag " + std::to_string(herr));
     }
-    const int e = job->spp_end ? job->spp_end : job->spp_x * job->spp_y;
-    const float inv = 1.f / (float)(e - job->spp_begin);
-    for (size_t i = 0; i < nf; ++i) film_rgb[i] *= inv;
   });
 }
 

@@ -227,6 +227,9 @@ __global__ void k_sort_hist(SceneView S, Queues Q, int qsel) {
   for (int b = threadIdx.x; b < PT_SORT_BINS; b += blockDim.x) h[b] = 0;
   __syncthreads();
   const int n = Q.counts[qsel];
+  // the bounce's traversal and the last one's shadow terms are done: counters
+  // of the next ray queue, the shadow queue and both fetches
+  if (blockIdx.x == 0 && threadIdx.x < 6 && (int)threadIdx.x != qsel) Q.counts[threadIdx.x] = 0;
   const int lane = threadIdx.x & 31;
   const int stride = gridDim.x * blockDim.x;
   const int nround = (n + stride - 1) / stride * stride;
@@ -359,6 +362,16 @@ __global__ void k_gaussian_blur(const float *in, float *out, int W, int H, int K
   }
 }
 
+// film *= inv: the mean from the sum of a render's samples (the last step of
+// pt_render's pixel loop, renderManager.hpp:115).
+__global__ void k_film_scale(float *film, float inv, long long n) {
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    film[i] = __fmul_rn(film[i], inv);
+}
+void launch_film_scale(float *film, float inv, long long n, cudaStream_t st) {
+  k_film_scale<<<grid_for(n, 256, 152 * 8), 256, 0, st>>>(film, inv, n);
+}
+
 // FrameBuffer::writeToFile pixel path (framebuffer.cpp:27-58).
 __global__ void k_tonemap(const float *film, int W, int H, float inv_gamma, uint8_t *out) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < W * H * 3; t += gridDim.x * blockDim.x) {
@@ -471,7 +484,6 @@ void launch_wave(const SceneView &S, const DeviceJob &J, const Queues &Q, long l
 }
 
 void launch_sort(const SceneView &S, const Queues &Q, int qsel, const LaunchCfg &cfg, cudaStream_t st) {
-  cudaMemsetAsync(Q.bins, 0, sizeof(int) * 2 * PT_SORT_BINS, st);
   k_sort_hist<<<cfg.max_blocks_simple, 256, 0, st>>>(S, Q, qsel);
   k_sort_scatter<<<cfg.max_blocks_simple, 256, 0, st>>>(Q, qsel);
 }

@@ -205,6 +205,7 @@ int persistent_grid(const SceneView &S, int num_sms);
 cudaError_t launch_group_persistent(const SceneView &S, const JobTable &T, const Queues &Q, float *const *d_films,
                                     long long total, int wave, int LN, int bounces, void *d_barrier, int grid,
                                     cudaStream_t st);
+void launch_film_scale(float *film, float inv, long long n, cudaStream_t st);
 void launch_tonemap(const float *film, int W, int H, float gamma, uint8_t *out, cudaStream_t st);
 void launch_gaussian_blur(const float *in, float *out, int W, int H, int K, const float *w, cudaStream_t st);
 

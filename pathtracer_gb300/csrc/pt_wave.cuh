@@ -307,9 +307,12 @@ __device__ __forceinline__ void camera_body(const DeviceJob &J0, const JobTable 
     Q.beta[s] = make_float4(1.f, 1.f, 1.f, -1.f);  // w < 0: previous vertex delta / camera
     Q.L[s] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    Q.counts[0] = n;
-    atomicAdd(&Q.stats[0], (unsigned long long)n);
+  if (blockIdx.x == 0 && threadIdx.x < 2 * PT_SORT_BINS) {
+    // the counters of the first bounce; k_sort_hist and k_sample clear them for
+    // the later ones (a memset between two kernels takes 2-3 us of a bounce)
+    Q.bins[threadIdx.x] = 0;
+    if (threadIdx.x < 6) Q.counts[threadIdx.x] = threadIdx.x == 0 ? n : 0;
+    if (threadIdx.x == 0) atomicAdd(&Q.stats[0], (unsigned long long)n);
   }
 }
 template <bool MJ>
@@ -699,6 +702,7 @@ template <bool MJ>
 __global__ void __launch_bounds__(256) k_sample(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel, int bounce,
                                                 long long g0) {
   const int ns = Q.seg[PT_FAM_MISC], m0 = Q.seg[PT_KEY_MEDIUM], nm = Q.seg[PT_KEY_MEDIUM + 1] - m0;
+  if (blockIdx.x == 0 && threadIdx.x < 2 * PT_SORT_BINS) Q.bins[threadIdx.x] = 0;  // for the next bounce's sort
   const bool med = S.has_medium != 0;
   const int first = (med ? 4 : 3) * bounce;  // the bounce's first dimension
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * ns + 2 * nm; t += gridDim.x * blockDim.x) {
@@ -1104,15 +1108,16 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
   auto paired = [&](int b) { return b > 0 && b < bounces && (n <= cfg.pair_trace || b >= from); };
   for (int b = 0; b < bounces; ++b) {
     const bool pair = paired(b);
-    // reset next-queue and fetch counters (device side, graph friendly)
     // ([2] shadow queue, [3] shadow fetch, [4] closest-hit fetch, [5] listed
-    // shadow rays); a pending shadow queue of the previous bounce keeps [2]
-    // and [5]
-    cudaMemsetAsync(Q.counts + (qsel ^ 1), 0, sizeof(int), st);
-    if (!pair)
-      cudaMemsetAsync(Q.counts + 2, 0, 4 * sizeof(int), st);
-    else
-      cudaMemsetAsync(Q.counts + 4, 0, sizeof(int), st);
+    // shadow rays) are cleared by k_camera and k_sort_hist; without the sort,
+    // here: a pending shadow queue of the previous bounce keeps [2] and [5]
+    if (!cfg.sort_by_material && b > 0) {
+      cudaMemsetAsync(Q.counts + (qsel ^ 1), 0, sizeof(int), st);
+      if (!pair)
+        cudaMemsetAsync(Q.counts + 2, 0, 4 * sizeof(int), st);
+      else
+        cudaMemsetAsync(Q.counts + 4, 0, sizeof(int), st);
+    }
     P.begin(STAGE_TRACE, st);
     if (pair) {
       // this bounce's closest rays with the previous bounce's shadow rays
@@ -1132,7 +1137,7 @@ void launch_wave_stages(const SceneView &S, const DeviceJob &J, const JobTable &
       // the previous bounce's shadow terms, before this bounce's shading
       P.begin(STAGE_SHADOW, st);
       launch_shadow_resolve(Q, LN, cfg, st);
-      cudaMemsetAsync(Q.counts + 2, 0, 4 * sizeof(int), st);
+      if (!cfg.sort_by_material) cudaMemsetAsync(Q.counts + 2, 0, 4 * sizeof(int), st);
       P.end(st);
       P.count(STAGE_SHADOW, 1);
     }
