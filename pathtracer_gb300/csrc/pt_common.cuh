@@ -336,11 +336,42 @@ struct OwenDigits {
   uint32_t a;    // the index's digits not yet taken
   uint64_t rev;  // the scrambled digits so far, most significant first
 };
-template <bool BASE2>
+// Bases by the mask w = fill_mask(base) of Kensler's permutation: only the
+// bits of w of every intermediate value reach the result, and for w <= 127 two
+// of the mixing steps vanish ((i & w) >> 11) or fold into the next product;
+// with w < 16 also (i & w) >> 4, with w < 32 the final i >> 5.
+enum OwenClass { OWEN_BASE2 = 0, OWEN_W15, OWEN_W31, OWEN_W127 };
+template <int C>
+PT_HD uint32_t permutation_prime(uint32_t i, uint32_t l, uint32_t w, uint32_t p) {
+  const uint32_t m = (1u | p >> 27) * (0x6935fa69u * 0x74dcb303u);
+  const uint32_t w1 = w >> 1, w2 = w >> 2;
+  do {
+    i ^= p;
+    i *= 0xe170893du;
+    if (C == OWEN_W15) {
+      i ^= (p >> 16) ^ (p >> 8);
+    } else {
+      i ^= p >> 16;
+      i ^= ((i & w) >> 4) ^ (p >> 8);
+    }
+    i *= 0x0929eb3fu;
+    i ^= p >> 23;
+    i ^= (i >> 1) & w1;
+    i *= m;
+    i ^= (i >> 2) & w2;
+    i *= 0x9e501cc3u;
+    i ^= (i >> 2) & w2;
+    i *= 0xc860a3dfu;
+    i &= w;
+    if (C == OWEN_W127) i ^= i >> 5;
+  } while (i >= l);
+  return i;
+}
+template <int C>
 PT_HD void owen_digit(const HaltonTables &T, int bi, uint32_t base, uint32_t w, uint32_t hash, int di,
                       OwenDigits &s) {
   const uint32_t dh = (uint32_t)mix_bits(hash ^ (uint32_t)s.rev ^ ((uint32_t)di << 16));
-  if (BASE2) {
+  if (C == OWEN_BASE2) {
     // permutation_element(d, 2, p) = d ^ bit 0 of (p >> 8 ^ p >> 16 ^ p >> 23):
     // with w = 1 every odd multiplier keeps bit 0, every (i & w) >> k
     // shift is 0, the loop runs once and the final + p cancels p's bit 0
@@ -352,7 +383,7 @@ PT_HD void owen_digit(const HaltonTables &T, int bi, uint32_t base, uint32_t w, 
     const uint32_t next = div_prime(T, bi, s.a);
     const uint32_t digit = s.a - next * base;
     // permutation_element(digit, base, dh), its modulo by the base's divisor
-    const uint32_t v = permutation_index(digit, base, w, dh) + dh;
+    const uint32_t v = permutation_prime<C>(digit, base, w, dh) + dh;
     s.rev = s.rev * base + (v - div_prime(T, bi, v) * base);
     s.a = next;
   }
@@ -361,7 +392,7 @@ PT_HD void owen_digit(const HaltonTables &T, int bi, uint32_t base, uint32_t w, 
 // modulo T.owen_pow only: `first`, the dimension's table by that remainder (or
 // null), gives them with one load in place of 2 (base 97) to 17 (base 2) of the
 // 6 to 38 digits up to the early end.
-template <bool BASE2>
+template <int C>
 PT_HD float owen_digits(const HaltonTables &T, int bi, uint32_t hash, uint32_t index, const uint32_t *first) {
   const uint32_t base = (uint32_t)T.prime[bi];
   const uint32_t w = fill_mask(base);
@@ -374,11 +405,11 @@ PT_HD float owen_digits(const HaltonTables &T, int bi, uint32_t hash, uint32_t i
     s.rev = first[index - s.a * T.owen_pow[bi]];
     di = T.owen_first[bi];
   }
-  for (; di < nc; ++di) owen_digit<BASE2>(T, bi, base, w, hash, di, s);
+  for (; di < nc; ++di) owen_digit<C>(T, bi, base, w, hash, di, s);
   const uint64_t lo = s.rev * T.owen_tail[bi];
   const float flo = clamp_to_float(xdmul(scale, (double)lo));
   if (flo == clamp_to_float(xdmul(scale, (double)(lo + (T.owen_tail[bi] - 1))))) return flo;
-  for (; di < nd; ++di) owen_digit<BASE2>(T, bi, base, w, hash, di, s);
+  for (; di < nd; ++di) owen_digit<C>(T, bi, base, w, hash, di, s);
   return clamp_to_float(xdmul(scale, (double)s.rev));
 }
 // The scrambling of dimension dim (sampler.hpp:69-71).
@@ -389,8 +420,11 @@ PT_HD float owen_radical_inverse(const HaltonTables &T, int dim, uint32_t index,
   const int bi = dim % PT_PRIME_COUNT;
   const uint32_t hash = owen_hash(dim);
   const uint32_t *first = tables && dim < PT_OWEN_DIMS ? tables + T.owen_at[dim] : nullptr;
-  return T.prime[bi] == 2 ? owen_digits<true>(T, bi, hash, index, first)
-                          : owen_digits<false>(T, bi, hash, index, first);
+  const int p = T.prime[bi];
+  if (p == 2) return owen_digits<OWEN_BASE2>(T, bi, hash, index, first);
+  if (p < 16) return owen_digits<OWEN_W15>(T, bi, hash, index, first);
+  if (p < 32) return owen_digits<OWEN_W31>(T, bi, hash, index, first);
+  return owen_digits<OWEN_W127>(T, bi, hash, index, first);
 }
 // Entry r of dimension dim's table.
 PT_HD uint32_t owen_first_digits(const HaltonTables &T, int dim, uint32_t r) {
@@ -398,8 +432,10 @@ PT_HD uint32_t owen_first_digits(const HaltonTables &T, int dim, uint32_t r) {
   const uint32_t base = (uint32_t)T.prime[bi], w = fill_mask(base), hash = owen_hash(dim);
   OwenDigits s{r, 0};
   for (int di = 0; di < T.owen_first[bi]; ++di) {
-    if (base == 2) owen_digit<true>(T, bi, base, w, hash, di, s);
-    else owen_digit<false>(T, bi, base, w, hash, di, s);
+    if (base == 2) owen_digit<OWEN_BASE2>(T, bi, base, w, hash, di, s);
+    else if (base < 16) owen_digit<OWEN_W15>(T, bi, base, w, hash, di, s);
+    else if (base < 32) owen_digit<OWEN_W31>(T, bi, base, w, hash, di, s);
+    else owen_digit<OWEN_W127>(T, bi, base, w, hash, di, s);
   }
   return (uint32_t)s.rev;
 }

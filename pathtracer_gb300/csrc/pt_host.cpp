@@ -921,9 +921,11 @@ static void collapse(const Builder &B, int bn, Bvh4Out &out, int depth, int me, 
 // ray's stack would not hold the deeper tree.  Shadow rays of the Cornell box
 // 6.42 -> 5.72 ms, hair on curves (paired launches) 4.42 -> 3.58, material
 // divergence 24.5 -> 24.1; one mesh alone does not change.  128 / 512 / 2048
-// units: Cornell 5.73 / 5.72 / 5.59, hair 4.05 / 3.58 / 3.57 (202 objects); the
-// sweep takes 0.3 ms of an upload at 256.
-// Subtrees and leaves an any-hit top groups.
+// units: Cornell 5.73 / 5.72 / 5.59, hair 4.05 / 3.58 / 3.57 (202 objects); 64
+// units for the Cornell box's 7 objects: the same 5.60 as 256, and 0.1 ms less
+// of its upload.
+// Subtrees and leaves an any-hit top groups at most (4 per object, 64 at
+// least: what few objects gain is gained at their first levels).
 #define PT_TOP_UNITS 256
 struct TopUnit {
   Box box;
@@ -1740,16 +1742,24 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   } freed{staged};
   int any_root = 0;
   if (device) {
-    // packed on the device; the host tree and its hash keep the float boxes
-    const std::vector<Bvh4Node> top = any_hit_top(out, PT_TOP_UNITS);
+    // the host tree and its hash keep the float boxes
+    const std::vector<Bvh4Node> top = any_hit_top(out, std::min(PT_TOP_UNITS, std::max(64, 4 * d->n_objects)));
     any_root = top.empty() ? 0 : (int)out.nodes.size();
-    const Bvh4Node *wide = dupload(out.nodes, staged, st), *wide_top = dupload(top, staged, st);
-    void *packed = nullptr;
-    cuda_check(cudaMalloc(&packed, sizeof(PackedNode) * (out.nodes.size() + top.size())), "cudaMalloc(nodes)");
-    S->owned.push_back(packed);
-    S->nodes = static_cast<PackedNode *>(packed);
-    launch_pack_nodes(wide, (int)out.nodes.size(), S->nodes, st);
-    if (!top.empty()) launch_pack_nodes(wide_top, (int)top.size(), S->nodes + out.nodes.size(), st);
+    const size_t nn = out.nodes.size() + top.size();
+    if (nn <= 4096) {  // packed here: two allocations on the device would take longer
+      std::vector<PackedNode> packed(nn);
+      for (size_t k = 0; k < nn; ++k)
+        packed[k] = pack_node(k < out.nodes.size() ? out.nodes[k] : top[k - out.nodes.size()]);
+      S->nodes = up(packed);
+    } else {
+      const Bvh4Node *wide = dupload(out.nodes, staged, st), *wide_top = dupload(top, staged, st);
+      void *packed = nullptr;
+      cuda_check(cudaMalloc(&packed, sizeof(PackedNode) * nn), "cudaMalloc(nodes)");
+      S->owned.push_back(packed);
+      S->nodes = static_cast<PackedNode *>(packed);
+      launch_pack_nodes(wide, (int)out.nodes.size(), S->nodes, st);
+      if (!top.empty()) launch_pack_nodes(wide_top, (int)top.size(), S->nodes + out.nodes.size(), st);
+    }
   }
   S->items = up(items);
   S->shade = up(shade);
@@ -1850,6 +1860,7 @@ Context::Context(int dev) : device(dev) {
   upload_halton_tables(halton, stream);
   upload_halton_tables_multi(halton, stream);
   upload_halton_tables_persist(halton, stream);
+  cuda_check(cudaMallocHost(&pinned, sizeof(Pinned)), "cudaMallocHost");
   cuda_check(cudaMalloc(&d_owen, sizeof(uint32_t) * halton.owen_at[PT_OWEN_DIMS]), "cudaMalloc(owen tables)");
   launch_owen_tables(d_owen, halton.owen_at[PT_OWEN_DIMS], stream);
   kernel_attributes(&kinfo);
@@ -1900,6 +1911,7 @@ Context::~Context() {
   if (d_scratch) cudaFree(d_scratch);
   if (d_err) cudaFree(d_err);
   if (d_owen) cudaFree(d_owen);
+  if (pinned) cudaFreeHost(pinned);
   for (cudaEvent_t e : prof.pool) cudaEventDestroy(e);
   if (stream) cudaStreamDestroy(stream);
 }
@@ -2087,7 +2099,8 @@ DeviceJob Context::device_job(const pt_job_desc &j, Scene *S) {
   return J;
 }
 
-void Context::render_device(const pt_job_desc &j, float *d_film, pt_stats *stats, bool sync, const float *d_rays) {
+void Context::render_device(const pt_job_desc &j, float *d_film, pt_stats *stats, bool sync, const float *d_rays,
+                            float *host_film, float scale) {
   validate_job(j);
   Scene *S = scene(j.scene);
   DeviceJob J = device_job(j, S);
@@ -2146,23 +2159,29 @@ void Context::render_device(const pt_job_desc &j, float *d_film, pt_stats *stats
   }
   cudaEventRecord(e1, stream);
   cuda_check(cudaGetLastError(), "launch");
-  if (sync || stats) {
+  const size_t nf = (size_t)npix * 3;
+  if (host_film) {
+    // the mean of the samples, then the film, behind the render
+    if (scale != 1.f) launch_film_scale(d_film, scale, (long long)nf, stream);
+    cuda_check(cudaMemcpyAsync(host_film, d_film, nf * sizeof(float), cudaMemcpyDeviceToHost, stream), "film d2h");
+  }
+  if (sync || stats || host_film) {
+    // error flag and counts by the same wait, into page-locked memory
+    cuda_check(cudaMemcpyAsync(&pinned->err, d_err, sizeof(int), cudaMemcpyDeviceToHost, stream), "read err");
+    if (stats) {
+      cuda_check(cudaMemcpyAsync(pinned->stats[0], Q.stats, 32, cudaMemcpyDeviceToHost, stream), "read stats");
+      if (waves > 1)
+        cuda_check(cudaMemcpyAsync(pinned->stats[1], Q2.stats, 32, cudaMemcpyDeviceToHost, stream), "read stats");
+    }
     cuda_check(cudaStreamSynchronize(stream), "render");
-    int herr = 0;
-    cuda_check(cudaMemcpy(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost), "read err");
-    if (herr) {
+    if (const int herr = pinned->err) {
       cudaMemset(d_err, 0, sizeof(int));
       fail(PT_ERR_DEVICE, "device traversal error flag " + std::to_string(herr));
     }
   }
   if (stats) {
     unsigned long long h[4];
-    cuda_check(cudaMemcpy(h, Q.stats, sizeof h, cudaMemcpyDeviceToHost), "read stats");
-    if (waves > 1) {
-      unsigned long long h2[4];
-      cuda_check(cudaMemcpy(h2, Q2.stats, sizeof h2, cudaMemcpyDeviceToHost), "read stats");
-      for (int k = 0; k < 4; ++k) h[k] += h2[k];
-    }
+    for (int k = 0; k < 4; ++k) h[k] = pinned->stats[0][k] + (waves > 1 ? pinned->stats[1][k] : 0);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
     stats->paths = h[0];
@@ -2410,18 +2429,8 @@ int pt_render(void *ctx, const pt_job_desc *job, float *film_rgb, pt_stats *stat
     const size_t nf = (size_t)job->width * job->height * 3;
     float *df = c->film_buffer(nf);
     cuda_check(cudaMemsetAsync(df, 0, nf * sizeof(float), c->stream), "memset film");
-    c->render_device(*job, df, stats, false);
-    // the mean, on the device (a 1080p film took the host 2 ms)
     const int e = job->spp_end ? job->spp_end : job->spp_x * job->spp_y;
-    launch_film_scale(df, 1.f / (float)(e - job->spp_begin), (long long)nf, c->stream);
-    cuda_check(cudaMemcpyAsync(film_rgb, df, nf * sizeof(float), cudaMemcpyDeviceToHost, c->stream), "film d2h");
-    cuda_check(cudaStreamSynchronize(c->stream), "render");
-    int herr = 0;
-    cuda_check(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read err");
-    if (herr) {
-      cudaMemset(c->d_err, 0, sizeof(int));
-      fail(PT_ERR_DEVICE, "device traversal error flag " + std::to_string(herr));
-    }
+    c->render_device(*job, df, stats, false, nullptr, film_rgb, 1.f / (float)(e - job->spp_begin));
   });
 }
 
@@ -2461,15 +2470,7 @@ int pt_ray_color(void *ctx, const pt_job_desc *job, const float *rays, int32_t n
     float *dr = (float *)c->scratch(nn * 24);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
     cuda_check(cudaMemsetAsync(df, 0, nn * 12, c->stream), "memset film");
-    c->render_device(j, df, nullptr, false, dr);
-    cuda_check(cudaMemcpyAsync(radiance, df, nn * 12, cudaMemcpyDeviceToHost, c->stream), "d2h");
-    cuda_check(cudaStreamSynchronize(c->stream), "ray color");
-    int herr = 0;
-    cuda_check(cudaMemcpy(&herr, c->d_err, sizeof(int), cudaMemcpyDeviceToHost), "read err");
-    if (herr) {
-      cudaMemset(c->d_err, 0, sizeof(int));
-      fail(PT_ERR_DEVICE, "device traversal error flag " + std::to_string(herr));
-    }
+    c->render_device(j, df, nullptr, false, dr, radiance, 1.f);
   });
 }
 

@@ -157,7 +157,13 @@ struct Context {
   // d_rays (device, 6 floats per film pixel): given primary rays instead of
   // the camera's (pt_ray_color)
   void render_device(const pt_job_desc &j, float *d_film, pt_stats *stats, bool sync,
-                     const float *d_rays = nullptr);
+                     const float *d_rays = nullptr, float *host_film = nullptr, float scale = 1.f);
+  // what a render reads back with its film
+  struct Pinned {
+    unsigned long long stats[2][4];
+    int err;
+  };
+  Pinned *pinned = nullptr;
   float *film_buffer(size_t floats);
   void *scratch(size_t bytes);
 };

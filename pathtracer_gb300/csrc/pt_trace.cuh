@@ -283,7 +283,7 @@ struct WarpHits {
   int32_t who[32];     // tester whose hit the owner takes
 };
 // Lanes (of 32) below which a walk pauses to see whether others have ended.
-#define PT_WALK_MIN 12
+#define PT_WALK_MIN 8
 // One kernel per kind of scene: PT_BY_SCENE(S, RUN) expands RUN(CURVES, MOTION).
 #define PT_BY_SCENE(S, RUN)          \
   do {                               \
@@ -483,15 +483,16 @@ __device__ __forceinline__ int warp_lanes(int n) {
 // active threads per instruction in the shadow kernel, 8.29 -> 6.66 ms for
 // its 51 M rays (with the compact ray list, PT_FETCH_IDLE_SHADOW 16).  Rough
 // glass, 16.8 M paths: trace 16.5 -> 13.8 ms (39 M rays), shadow 16.8 ->
-// 13.3 ms (45 M).  Testing from 24 / 16 leaves on: shadow 13.0 / 13.1 ms on
-// the glass, 6.75 / 7.16 on Cornell, so 32 stays.  With 32 lanes always (no
+// 13.3 ms (45 M).  Testing from 24 leaves on instead of 32 takes any-hit rays
+// 23.9 -> 23.2 ms on the material divergence and 5.68 -> 5.62 on Cornell (they
+// end sooner); from 20 on 23.9 and 5.69; closest hits +0.4 % at 24, so 32 there.  With 32 lanes always (no
 // even share) bounces of few rays wait for each other's leaves: the
 // 0.48 M-path glass frame 3.57 -> 3.9 ms.
 //
 // A turn of the walk does one node visit; done rays and the refill are looked at
 // only when PT_WALK_MIN lanes or fewer still walk (rough glass trace 12.9 ->
-// 12.2 ms, shadow 11.5 -> 10.6 against a look every turn; 8 / 16 / 20 lanes are
-// within 1 % but for closest hits at 20, +3 %).  MOTION = false (scenes without
+// 12.2 ms, shadow 11.5 -> 10.6 against a look every turn; 8 / 12 / 16 lanes are
+// within 1 %, closest hits at 20 +3 %).  MOTION = false (scenes without
 // moving objects) compiles the changes of frame out: trace 11.4 -> 10.9 ms, the
 // 0.48 M-path glass frame's 1.60 -> 1.49.
 //
@@ -580,7 +581,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
     // ---- walk: leaves reached go to the list, a node visit for every lane
     // that stands at one; until the list is full, or so few lanes walk on that
     // others may have ended
-    const int full = min(32, in_flight);
+    const int full = min(MODE == TRACE_ANY ? 24 : 32, in_flight);
     unsigned rm;
     for (;;) {
       const bool leaf = active && ref_is_leaf(R.ref);

@@ -696,8 +696,9 @@ __device__ __forceinline__ void list_shadow_rays(const Queues &Q, unsigned lit, 
 // kernel and runs it at 3 times their occupancy; with the tables of first
 // digits (owen_digits) rough glass shades 16.8 M paths in 13.1 ms instead of
 // 15.0, the Cornell frame in 6.2 instead of 7.3 (2^15 / 2^20 entries per table:
-// 13.4 / 12.8 ms; 2^17 keeps all 64 tables at 12 MB), and 12.9 / 6.0 with the
-// early end tested from b^k >= 2^35 instead of 2^38.
+// 13.4 / 12.8 ms; 2^17 keeps all 64 tables at 12 MB), 12.9 / 6.0 with the early
+// end tested from b^k >= 2^35 instead of 2^38, and 12.0 / 5.6 (from 12.6 / 5.95)
+// with the permutation's vanishing steps left out and one thread per vertex.
 template <bool MJ>
 __global__ void __launch_bounds__(256) k_sample(SceneView S, DeviceJob J, JobTable T, Queues Q, int qsel, int bounce,
                                                 long long g0) {
@@ -705,19 +706,26 @@ __global__ void __launch_bounds__(256) k_sample(SceneView S, DeviceJob J, JobTab
   if (blockIdx.x == 0 && threadIdx.x < 2 * PT_SORT_BINS) Q.bins[threadIdx.x] = 0;  // for the next bounce's sort
   const bool med = S.has_medium != 0;
   const int first = (med ? 4 : 3) * bounce;  // the bounce's first dimension
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * ns + 2 * nm; t += gridDim.x * blockDim.x) {
-    const bool surf = t < 3 * ns;
-    const int u = surf ? t : t - 3 * ns, n = surf ? ns : nm;
-    const int d = (u >= n) + (surf && u >= 2 * n);
-    const int ii = u - d * n + (surf ? 0 : m0);
-    const int path = __float_as_int(ld4(Q.ray_o[qsel] + Q.order[ii]).w);
+  // a thread per dimension while the grid has threads for all, else one per
+  // vertex (which reads the vertex's path and finds its index once)
+  const int stride = gridDim.x * blockDim.x;
+  const bool split = 3 * ns + 2 * nm <= stride;
+  const int ts = split ? 3 * ns : ns, total = ts + (split ? 2 * nm : nm);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += stride) {
+    const bool surf = t < ts;
+    const int u = surf ? t : t - ts, n = surf ? ns : nm;
+    const int d0 = split ? (u >= n) + (surf && u >= 2 * n) : 0, d1 = split ? d0 + 1 : (surf ? 3 : 2);
+    const int ii = u - d0 * n + (surf ? 0 : m0);
+    const int path = __float_as_int(__ldg(&Q.ray_o[qsel][Q.order[ii]].w));
     long long g;
     const DeviceJob &Jp = path_job<MJ>(J, T, Q, path, g0, g);
     if (bounce >= Jp.job.max_depth) continue;  // nothing is sampled there
     const PathId P = path_id(Jp, g);
-    const int dim = first + (surf ? (med ? 1 : 0) : 2) + d;
-    Q.smp[(size_t)d * Q.cap + ii] = sampler_dim(Jp, dim, P.halton_index, P.key, P.pix, P.k);
-    if (d == 0) Q.smp_key[ii] = P.key;
+    const int dim = first + (surf ? (med ? 1 : 0) : 2);
+#pragma unroll 1
+    for (int d = d0; d < d1; ++d)
+      Q.smp[(size_t)d * Q.cap + ii] = sampler_dim(Jp, dim + d, P.halton_index, P.key, P.pix, P.k);
+    if (d0 == 0) Q.smp_key[ii] = P.key;
   }
 }
 
