@@ -58,7 +58,7 @@ FALLBACK_HBM_GBS = 6800.0
 # traversal-stage launches (closest, paired, shadow and the shadow resolve) of
 # one step of 16 spp of every pixel, per (workload, estimator); from a
 # one-pass ncu capture of the same bench command
-NCU_TRAVERSAL_BYTES_PER_STEP = {("rough_glass", 0): 8.850e9}
+NCU_TRAVERSAL_BYTES_PER_STEP = {("rough_glass", 0): 7.151e9}
 # Algorithmic queue bytes per unit, by stage: the records each stage must
 # read or write in this layout -- 192 B per path vertex,
 # 88 B per shadow ray (44 written by shade, 44 read by the traversal) and FP32
@@ -813,8 +813,8 @@ def run_ours(args, rank, world, local_rank):
                                           ("shadow_rays", "shadow"), ("film_pixel_waves", "film_pixel_waves"))},
                      "note": f"stage share {dom_ms / sum(v[0] for v in prof.values()):.2f}; "
                              f"whole-step queue bytes (192 B per vertex + 88 B per shadow ray + 24 B per path) "
-                             f"{step_bytes_gbs:.1f} GB/s; the traversal is bound by dependent node-load "
-                             "latency, not bandwidth (L2 hit rate and warp efficiency in the committed ncu summary)"},
+                             f"{step_bytes_gbs:.1f} GB/s; the traversal is bound by instruction issue "
+                             "and divergence, not bandwidth (issue and warp efficiency in the committed ncu summary)"},
         "stage_ms": {kk: round(v[0], 3) for kk, v in prof.items()},
         "clocks": clk.summary(),
         "wall_s": wall,

@@ -3,8 +3,9 @@
 // the batch test kernels behind the C-ABI.
 //
 // One wave = a contiguous range of (sample, pixel) paths.  Per bounce:
-//   k_trace_closest  RayQueue -> HitQueue            (BVH4, shared-mem stack)
+//   k_trace_closest  RayQueue -> HitQueue            (packed BVH4, warp-wide leaf list)
 //   k_sort_*         HitQueue -> order by material family (counting sort)
+//   k_sample         order -> sampler dimensions and keys of the sorted vertices
 //   k_shade<FAM>     logic + BSDF sample + NEE: writes next RayQueue
 //                    (warp-aggregated compaction) and ShadowQueue
 //   k_trace_shadow   ShadowQueue any-hit visibility
