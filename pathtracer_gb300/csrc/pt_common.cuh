@@ -47,6 +47,22 @@ PT_HD float xsqrt(float a) { return std::sqrt(a); }
 PT_HD double xdmul(double a, double b) { return a * b; }
 #endif
 
+// x / n for a small whole number n whose rounded reciprocal r is at hand:
+// Markstein's correction of the product (IBM J. R&D 34, 1990) gives the
+// rounded quotient, without a division's range checks.  x normal or zero.
+PT_HD float div_small(float x, float n, float r) {
+#if defined(__CUDA_ARCH__)
+  const float q = __fmul_rn(x, r);
+  return __fmaf_rn(__fmaf_rn(-q, n, x), r, q);
+#else
+  const float q = x * r;
+  return std::fma(std::fma(-q, n, x), r, q);
+#endif
+}
+// a / b for 0 <= a < 16, 0 < b <= 16, r = 1 / b: (a + 1/2) / b is at least
+// 1/32 from a whole number.
+PT_HD int idiv_small(int a, float r) { return (int)(((float)a + 0.5f) * r); }
+
 // sin/cos of pi*x and of x (device intrinsics; libm on the host).
 PT_HD void sincospi_(float x, float *s, float *c) {
 #if defined(__CUDA_ARCH__)

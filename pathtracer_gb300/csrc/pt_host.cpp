@@ -1764,6 +1764,7 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   S->items = up(items);
   S->shade = up(shade);
   S->materials = up(mats);
+  for (LightRec &L : lights) L.pdf = L.area <= 1e-7f ? 0.f : 1.f / (L.area * (float)lights.size());
   S->lights = up(lights);
   SceneView &V = S->view;
   std::memset(&V, 0, sizeof V);
@@ -2089,6 +2090,8 @@ DeviceJob Context::device_job(const pt_job_desc &j, Scene *S) {
   J.job.env_sampling = (S->view.env.present ? j.env_sampling : PT_ENV_UNIFORM);
   J.job.light_nx = j.light_samples_x;
   J.job.light_ny = j.light_samples_y;
+  J.job.inv_light_nx = 1.f / (float)j.light_samples_x;
+  J.job.inv_light_ny = 1.f / (float)j.light_samples_y;
   J.job.seed = j.seed;
   J.job.shutter = j.camera.shutter;
   J.job.cam = make_camera(j.camera);

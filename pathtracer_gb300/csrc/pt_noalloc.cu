@@ -122,6 +122,8 @@ void render_device_noalloc(Context *c, const pt_job_desc &j, float *d_film, pt_s
   J.job.env_sampling = S->view.env.present ? j.env_sampling : PT_ENV_UNIFORM;
   J.job.light_nx = j.light_samples_x;
   J.job.light_ny = j.light_samples_y;
+  J.job.inv_light_nx = 1.f / (float)j.light_samples_x;
+  J.job.inv_light_ny = 1.f / (float)j.light_samples_y;
   J.job.seed = j.seed;
   J.job.shutter = j.camera.shutter;
   if (S->view.has_motion && j.camera.shutter > S->shutter_max)

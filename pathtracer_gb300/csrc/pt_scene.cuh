@@ -79,7 +79,7 @@ struct alignas(16) LightRec {
   float e1[3];      // quad: vertices[1] - vertices[0]
   int32_t motion;   // motion index + 1 (0: static)
   float e2[3];      // quad: vertices[3] - vertices[0]
-  float pad1;
+  float pdf;        // 1 / (area * number of lights): the density of a sample by area
   float normal[3];  // quad: normalize(cross(e1, e2))
   float pad2;
   float color[3];   // ConstantTexture colour
@@ -171,6 +171,7 @@ struct JobView {
   int32_t sampler;
   int32_t env_sampling;
   int32_t light_nx, light_ny;
+  float inv_light_nx, inv_light_ny;  // rounded reciprocals (div_small)
   uint32_t seed;
   float shutter;          // motion blur: a path's time is shutter * u
   CameraView cam;

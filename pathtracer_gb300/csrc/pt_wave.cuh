@@ -477,10 +477,15 @@ __device__ __forceinline__ float power_heuristic(float nf, float fpdf, float ng,
 // maxdepth_nee.hpp:91 draws per shading vertex, stratum (i, j) = (ls / ny,
 // ls % ny), i outer; the jitter from the path's counter stream at the
 // vertex's slot base rbase.
+// The grid's divisions, the light index's remainder and a light's density by
+// area were ~80 of a sample's ~470 instructions; as products by reciprocals
+// (exact: div_small, idiv_small), a subtraction and an uploaded constant they
+// take the Cornell frame's shading 5.60 -> 5.40 ms, the rough glass's 11.96 ->
+// 11.74 and the material divergence's 20.28 -> 19.94, with the same bits.
 __device__ __forceinline__ float2 light_offset(const DeviceJob &J, uint64_t key, uint32_t rbase, int ls) {
-  const int si = ls / J.job.light_ny, sj = ls % J.job.light_ny;
-  return make_float2(((float)si + rand01(key, rbase + 2u * ls)) / (float)J.job.light_nx,
-                     ((float)sj + rand01(key, rbase + 2u * ls + 1u)) / (float)J.job.light_ny);
+  const int si = idiv_small(ls, J.job.inv_light_ny), sj = ls - si * J.job.light_ny;
+  return make_float2(div_small((float)si + rand01(key, rbase + 2u * ls), (float)J.job.light_nx, J.job.inv_light_nx),
+                     div_small((float)sj + rand01(key, rbase + 2u * ls + 1u), (float)J.job.light_ny, J.job.inv_light_ny));
 }
 
 // A light sample seen from x (maxdepth_nee.hpp:104-189): the point of
@@ -595,7 +600,8 @@ __device__ __forceinline__ bool next_event(const SceneView &S, const DeviceJob &
   {
     const float2 lo = light_offset(J, key, rbase, ls);
     const float ox = lo.x, oy = lo.y;
-    int li = (int)(rand01(key, rbase + 20u + ls) * S.n_lights) % S.n_lights;
+    int li = (int)(rand01(key, rbase + 20u + ls) * S.n_lights);  // u < 1: at most n_lights, by rounding
+    if (li >= S.n_lights) li -= S.n_lights;
     const LightRec &Lr = S.lights[li];
     V3 wl, Le;
     float tmax, pdf_l, G, NoI, tr = 1.f;
@@ -624,7 +630,7 @@ __device__ __forceinline__ bool next_event(const SceneView &S, const DeviceJob &
       Le = P.Le;
       if (len < 0.001f) valid = false;
       tmax = len - 0.001f;
-      pdf_l = (Lr.area <= 1e-7f) ? 0.f : 1.f / (Lr.area * (float)S.n_lights);
+      pdf_l = Lr.pdf;
       NoI = MED ? 1.f : fmaxf(0.f, dot(sf.n, wl));
       float NoL = fmaxf(0.f, dot(ln, -wl));
       float d2 = len * len;
