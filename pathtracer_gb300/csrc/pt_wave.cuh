@@ -644,7 +644,7 @@ __device__ __forceinline__ bool next_event(const SceneView &S, const DeviceJob &
     }
     if (valid && G > 0.f) {
       V3 f;
-      float pb;
+      float pb = 0.f;
       if (MED) {
         f = v3(phase);
         pb = phase;
@@ -652,7 +652,7 @@ __device__ __forceinline__ bool next_event(const SceneView &S, const DeviceJob &
         // f and scatter_pdf: every BSDF in the shading normal's frame --
         // HairMarschner's too (hairMarsch.hpp:49, hairMarsch.cpp:115), even on
         // a curve, whose tangent only frames its sampling
-        bsdf_eval_t<FAM>(S.materials[mat], wo, wl, sf.n, sf.front, f, pb);
+        bsdf_eval_t<FAM>(S.materials[mat], wo, wl, sf.n, sf.front, mis, f, pb);
         if ((FAM == 0 || FAM < 0) && tex_alb) f = alb * PT_INV_PI_F;  // textured Lambertian albedo
       }
       float w = mis ? power_heuristic((float)LN, pdf_l, 1.f, pb) : 1.f;
