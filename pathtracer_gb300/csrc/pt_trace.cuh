@@ -48,9 +48,25 @@ __device__ __forceinline__ bool hit_triangle(const Item &it, V3 o, V3 d, float t
   return true;
 }
 
+// One axis of the test of a primitive's own bounds, for a t of 0 / 0 (the ray
+// lies in a rectangle's plane, or along a curve's axis).  Such a t passes every
+// comparison, so it is a hit wherever the primitive is tested: where the ray
+// meets its bounds, not wherever the traversal's boxes, which are rounded
+// outwards, let it through.
+__device__ __forceinline__ bool bounds_axis(float o, float d, float lo, float hi, float &near, float &far) {
+  if (d == 0.f) return !(o < lo || o > hi);
+  const float a = (lo - o) / d, b = (hi - o) / d;
+  near = fmaxf(near, fminf(a, b));
+  far = fminf(far, fmaxf(a, b));
+  return !(near > far);
+}
+// The far end of that test: a hit of the same leaf at the bounds may be tmax.
+__device__ __forceinline__ float bounds_far(float tmax) { return fmaf(fabsf(tmax), 0x1p-16f, tmax); }
+
 // AARectangle<axis>::intersect with the normalised direction dn.
-__device__ __forceinline__ bool hit_quad(const Item &it, V3 o, V3 dn, float tmin, float tmax,
-                                         float &t_out) {
+template <class Unordered>
+__device__ __forceinline__ bool hit_quad(const Item &it, V3 o, V3 dn, float tmin, float tmax, float &t_out,
+                                         Unordered unordered) {
   const int axis = (int)it.b[2];
   const float k = it.a[0], d0min = it.a[1], d0max = it.a[2];
   const float d1min = it.b[0], d1max = it.b[1];
@@ -64,6 +80,11 @@ __device__ __forceinline__ bool hit_quad(const Item &it, V3 o, V3 dn, float tmin
   }
   float t = xdiv(xsub(k, oa), da);
   if (t < tmin || t > tmax) return false;
+  if (t != t) {
+    unordered();
+    float near = tmin, far = bounds_far(tmax);
+    if (!bounds_axis(o0, d0_, d0min, d0max, near, far) || !bounds_axis(o1, d1_, d1min, d1max, near, far)) return false;
+  }
   float a0 = xadd(o0, xmul(t, d0_));
   float a1 = xadd(o1, xmul(t, d1_));
   if (a0 < d0min || a0 > d0max || a1 < d1min || a1 > d1max) return false;
@@ -145,6 +166,19 @@ __device__ __forceinline__ CurveSegment curve_segment(const float4 *cp, int i) {
   return g;
 }
 
+// Whether a ray meets a curve's bounds (Curve::getAABB, primitives/curve.hpp:
+// 33-46).  A function of its own: inlined, its registers spill those of the
+// curve kernels (hair trace 3.65 -> 3.71 ms).
+static __device__ __noinline__ bool meets_curve(const float4 *cp, V3 o, V3 d, float tmin, float tmax) {
+  const float4 a = __ldg(cp), b = __ldg(cp + 1), c = __ldg(cp + 2), e = __ldg(cp + 3);
+  const float r = fmaxf(a.w, b.w);
+  float near = tmin, far = bounds_far(tmax);
+  auto axis = [&](float oo, float dd, float p, float q, float s, float t) {
+    return bounds_axis(oo, dd, fminf(fminf(p, q), fminf(s, t)) - r, fmaxf(fmaxf(p, q), fmaxf(s, t)) + r, near, far);
+  };
+  return axis(o.x, d.x, a.x, b.x, c.x, e.x) && axis(o.y, d.y, a.y, b.y, c.y, e.y) && axis(o.z, d.z, a.z, b.z, c.z, e.z);
+}
+
 // Curve::intersect (primitives/curve.hpp:48-129) over the curve's segments
 // (8 x 32 B); roots from gl::solveQuadratic (utility.hpp:112-124).  Returns
 // the segment in u and the position along it in v (fraction of its length).
@@ -221,10 +255,10 @@ __device__ __forceinline__ V3 moved_origin(const SceneView &S, uint32_t motion, 
 // hit in [tmin, tmax] fills `hit`.  dn points at the ray's normalised
 // direction (rectangles and spheres read it).  CURVES = false compiles the
 // curve test out (curve items then never hit), MOTION = false the moving
-// primitives.
-template <bool CURVES, bool MOTION>
+// primitives.  unordered() is called for a hit of t = 0 / 0.
+template <bool CURVES, bool MOTION, class Unordered>
 __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V3 d, const float4 *dn4, float tmin,
-                                          float tmax, HitRec &hit, float time) {
+                                          float tmax, HitRec &hit, float time, Unordered unordered) {
   Item it = load_item(S.items, idx);
   const int type = (int)f2u(it.b[3]);
   const uint32_t motion = MOTION ? f2u(it.c[3]) : 0u;
@@ -235,11 +269,15 @@ __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V
     h = hit_triangle(it, o, d, tmin, tmax, t, u, v);
   } else if (CURVES && type == ITEM_CURVE) {
     h = hit_curve(S.curve_segments + 2 * PT_CURVE_SEGMENTS * (size_t)f2u(it.a[0]), o, d, tmin, tmax, t, u, v);
+    if (h && !(t <= tmax)) {  // along a segment's axis: a root of 0 / 0
+      h = meets_curve(S.curves + 4 * (size_t)__float_as_uint(__ldg(S.items[idx].a)), o, d, tmin, tmax);
+      unordered();
+    }
   } else if (type == ITEM_CURVE) {
     h = false;
   } else {
     const V3 dn = v3(dn4->x, dn4->y, dn4->z);
-    h = type == ITEM_QUAD ? hit_quad(it, o, dn, tmin, tmax, t) : hit_sphere(it, o, dn, tmin, tmax, t);
+    h = type == ITEM_QUAD ? hit_quad(it, o, dn, tmin, tmax, t, unordered) : hit_sphere(it, o, dn, tmin, tmax, t);
   }
   if (h) {
     hit.t = t;
@@ -279,9 +317,13 @@ struct WarpRays {
 // Closest-hit rays only: the nearest hit so far.
 struct WarpHits {
   float4 hit[32];      // t, prim (int bits, -1: none), u, v
-  uint32_t tmax[32];   // float_key of the ray's tmax
-  int32_t who[32];     // tester whose hit the owner takes
+  uint32_t tmax[32];   // float_key of the ray's tmax; PT_TMAX_STEPS: hit.x is its tmax
+  int32_t who[32];     // tester whose hit the owner takes, else one of PT_WHO_*
+  uint32_t again;      // lanes whose rays met a hit of no order (trace_rays)
 };
+#define PT_WHO_NONE (-1)   // a closest-hit ray
+#define PT_WHO_ANY (-2)    // an any-hit ray
+#define PT_TMAX_STEPS 0xffffffffu  // of a ray that is walked leaf by leaf (and of NaN)
 // Lanes (of 32) below which a walk pauses to see whether others have ended.
 #define PT_WALK_MIN 8
 // One kernel per kind of scene: PT_BY_SCENE(S, RUN) expands RUN(CURVES, MOTION).
@@ -478,6 +520,14 @@ __device__ __forceinline__ int warp_lanes(int n) {
 // are tested in the order it reached them, and of two equal-t hits the later
 // one wins, as in the reference's leaf loop.
 //
+// A hit of t = NaN (0 / 0: a ray in the plane of a rectangle; rays with NaN)
+// has no order: a leaf loop accepts it, and any hit after it, whatever its
+// distance (t > tmax is false with a NaN on either side).  A closest-hit ray
+// that meets one therefore starts again and is walked leaf by leaf, each leaf
+// tested before the walk goes on, which is that loop's order to the letter.
+// What this costs the others: rough glass trace 10.41 -> 10.58 ms, Cornell 2.71
+// -> 2.76, hair 3.56 -> 3.65.
+//
 // Measured against turns in which a warp either visits nodes or tests one item
 // per lane standing at a leaf (Cornell box, 256 x 256 x 64 spp): 15.3 -> 20.1
 // active threads per instruction in the shadow kernel, 8.29 -> 6.66 ms for
@@ -518,24 +568,45 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
   int iters = 0;
   bool active = false;     // the lane has a ray in flight
   bool pend = false;       // the list holds leaves of this lane's (last) ray
+  bool steps = false;      // its ray is walked leaf by leaf
   bool any = MODE == TRACE_ANY;
   bool exhausted = false;  // the queue has no unclaimed rays
   int qn = 0;              // leaves in the list
+  if (MODE != TRACE_ANY) {
+    if (lane == 0) H.again = 0;
+    __syncwarp();
+  }
   for (;;) {
     // ---- rays that ended: nothing left to visit or to test
-    if (active && !pend && R.ref == PT_REF_EMPTY && R.sp > 0) R.ref = K.pop(R.sp);
+    while (active && !pend && R.ref == PT_REF_EMPTY && R.sp > 0) R.ref = K.pop(R.sp);
     if (active && !pend && R.ref == PT_REF_EMPTY) {
-      HitRec h;
-      h.prim = -1;
-      if (MODE != TRACE_ANY) {
-        const float4 b = H.hit[lane];
-        h.t = b.x;
-        h.prim = __float_as_int(b.y);
-        h.u = b.z;
-        h.v = b.w;
+      if (MODE != TRACE_ANY && !steps && (H.again >> lane & 1u)) {
+        // start again, leaf by leaf
+        if (MOTION) {  // in the world's frame
+          const V3 o = v3(ow[0], ow[1], ow[2]);
+          W.o[lane] = make_float4(o.x, o.y, o.z, W.o[lane].w);
+          R.oi = v3(-o.x * R.inv.x, -o.y * R.inv.y, -o.z * R.inv.z);
+        }
+        R.tmax = W.dn[lane].w;
+        H.hit[lane] = make_float4(R.tmax, __int_as_float(-1), 0.f, 0.f);
+        H.tmax[lane] = PT_TMAX_STEPS;
+        R.ref = 0;
+        iters = 0;
+        steps = true;
+      } else {
+        HitRec h;
+        h.prim = -1;
+        if (MODE != TRACE_ANY) {
+          const float4 b = H.hit[lane];
+          h.t = b.x;
+          h.prim = __float_as_int(b.y);
+          h.u = b.z;
+          h.v = b.w;
+          if (steps) atomicAnd(&H.again, ~(1u << lane));
+        }
+        done(h.prim >= 0, h);
+        active = false;
       }
-      done(h.prim >= 0, h);
-      active = false;
     }
     // ---- refill
     const unsigned idle = __ballot_sync(0xffffffffu, !active && !pend);
@@ -557,9 +628,12 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           W.d[lane] = make_float4(d.x, d.y, d.z, R.tmin);
           W.dn[lane] = make_float4(dn.x, dn.y, dn.z, R.tmax);
           if (MODE != TRACE_ANY) {
-            H.hit[lane] = make_float4(FLT_MAX, __int_as_float(-1), 0.f, 0.f);
+            H.hit[lane] = make_float4(R.tmax, __int_as_float(-1), 0.f, 0.f);
             H.tmax[lane] = float_key(R.tmax);
-            H.who[lane] = any ? -2 : -1;  // -2: an any-hit ray
+            H.who[lane] = any ? PT_WHO_ANY : PT_WHO_NONE;
+            // what else has no order: rays that are not finite, or so far that
+            // a product of their coordinates is not
+            steps = !(fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + xdot(d, d) < 1e18f) || R.tmax != R.tmax;
           }
           if (MOTION) {
             ow[0] = o.x;
@@ -592,7 +666,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
         W.owner[at] = (uint8_t)lane;
         pend = true;
         ++iters;
-        R.ref = K.pop(R.sp);
+        R.ref = MODE != TRACE_ANY && steps ? PT_REF_EMPTY : K.pop(R.sp);  // popped when the leaf is tested
       }
       qn += __popc(lm);
       const bool ready = active && ref_is_node(R.ref) && !(MOTION && pend && ref_is_frame(R.ref));
@@ -646,14 +720,18 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
     if (lane < m) {
       const float4 o4 = W.o[own], d4 = W.d[own];
       float tm;
-      if (MODE == TRACE_MIXED) eany = H.who[own] == -2;
+      if (MODE == TRACE_MIXED) eany = H.who[own] == PT_WHO_ANY;
       if (MODE == TRACE_ANY) tm = W.dn[own].w;
-      else tm = key_float(H.tmax[own]);
+      else if (H.tmax[own] != PT_TMAX_STEPS) tm = key_float(H.tmax[own]);
+      else tm = H.hit[own].x;
       const V3 o = v3(o4.x, o4.y, o4.z), d = v3(d4.x, d4.y, d4.z);
       const int32_t code = ~lref;  // first_item << 3 | count - 1
       const int last = (code >> 3) + (code & 7);
+      auto unordered = [&] {
+        if (MODE != TRACE_ANY && !eany) atomicOr(&H.again, 1u << own);
+      };
       for (int i = code >> 3; i <= last; ++i) {
-        if (test_item<CURVES, MOTION>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w)) {
+        if (test_item<CURVES, MOTION>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w, unordered)) {
           hit = true;
           if (eany) break;
           tm = h.t;
@@ -692,7 +770,11 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
         __syncwarp();
         if (active && !any) {
           R.tmax = key_float(H.tmax[lane]);
-          H.who[lane] = -1;
+          H.who[lane] = PT_WHO_NONE;
+          if (steps) {
+            R.tmax = H.hit[lane].x;
+            H.tmax[lane] = PT_TMAX_STEPS;
+          }
         }
       }
     }
