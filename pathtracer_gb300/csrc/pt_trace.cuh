@@ -24,6 +24,26 @@ struct HitRec {
   float u, v;
 };
 
+// A hit of t = NaN: 0 / 0 of a ray in a rectangle's plane or along a straight
+// curve's axis.  It passes every comparison, so the reference's leaf loop takes
+// it where the ray meets the primitive's bounds, and after it any other hit: it
+// has no place in an order by t.  A closest-hit ray of trace_rays that meets one
+// is marked and walked again, leaf by leaf, in the leaf loop's own order.  Tests
+// that take such a hit (EXACT) ask whether the ray meets the primitive's own
+// bounds, since the packed boxes, rounded outwards, let more rays through.
+enum RayState : uint8_t { RAY_ORDERED = 0, RAY_MARKED = 1, RAY_ALONE = 2 };
+
+// One axis of that test; near and far: what is left of the ray.
+__device__ __forceinline__ bool bounds_axis(float o, float d, float lo, float hi, float &near, float &far) {
+  if (d == 0.f) return !(o < lo || o > hi);
+  const float a = (lo - o) / d, b = (hi - o) / d;
+  near = fmaxf(near, fminf(a, b));
+  far = fminf(far, fmaxf(a, b));
+  return !(near > far);
+}
+// Its far end: a hit of the same leaf on the bounds may be tmax.
+__device__ __forceinline__ float bounds_far(float tmax) { return fmaf(fabsf(tmax), 0x1p-16f, tmax); }
+
 // Moller-Trumbore exactly as hitTriangle orders it.
 __device__ __forceinline__ bool hit_triangle(const Item &it, V3 o, V3 d, float tmin, float tmax,
                                              float &t_out, float &u_out, float &v_out) {
@@ -48,25 +68,10 @@ __device__ __forceinline__ bool hit_triangle(const Item &it, V3 o, V3 d, float t
   return true;
 }
 
-// One axis of the test of a primitive's own bounds, for a t of 0 / 0 (the ray
-// lies in a rectangle's plane, or along a curve's axis).  Such a t passes every
-// comparison, so it is a hit wherever the primitive is tested: where the ray
-// meets its bounds, not wherever the traversal's boxes, which are rounded
-// outwards, let it through.
-__device__ __forceinline__ bool bounds_axis(float o, float d, float lo, float hi, float &near, float &far) {
-  if (d == 0.f) return !(o < lo || o > hi);
-  const float a = (lo - o) / d, b = (hi - o) / d;
-  near = fmaxf(near, fminf(a, b));
-  far = fminf(far, fmaxf(a, b));
-  return !(near > far);
-}
-// The far end of that test: a hit of the same leaf at the bounds may be tmax.
-__device__ __forceinline__ float bounds_far(float tmax) { return fmaf(fabsf(tmax), 0x1p-16f, tmax); }
-
 // AARectangle<axis>::intersect with the normalised direction dn.
-template <class Unordered>
+template <bool EXACT>
 __device__ __forceinline__ bool hit_quad(const Item &it, V3 o, V3 dn, float tmin, float tmax, float &t_out,
-                                         Unordered unordered) {
+                                         uint8_t *state) {
   const int axis = (int)it.b[2];
   const float k = it.a[0], d0min = it.a[1], d0max = it.a[2];
   const float d1min = it.b[0], d1max = it.b[1];
@@ -79,11 +84,15 @@ __device__ __forceinline__ bool hit_quad(const Item &it, V3 o, V3 dn, float tmin
     oa = o.z; da = dn.z; o0 = o.x; d0_ = dn.x; o1 = o.y; d1_ = dn.y;
   }
   float t = xdiv(xsub(k, oa), da);
-  if (t < tmin || t > tmax) return false;
-  if (t != t) {
-    unordered();
-    float near = tmin, far = bounds_far(tmax);
-    if (!bounds_axis(o0, d0_, d0min, d0max, near, far) || !bounds_axis(o1, d1_, d1min, d1max, near, far)) return false;
+  if (EXACT) {
+    if (t < tmin || t > tmax) return false;
+    if (t != t && da == 0.f) {
+      float near = tmin, far = bounds_far(tmax);
+      if (!bounds_axis(o0, d0_, d0min, d0max, near, far) || !bounds_axis(o1, d1_, d1min, d1max, near, far)) return false;
+    }
+  } else if (!(t >= tmin && t <= tmax)) {
+    if (t != t) *state = RAY_MARKED;
+    return false;
   }
   float a0 = xadd(o0, xmul(t, d0_));
   float a1 = xadd(o1, xmul(t, d1_));
@@ -167,8 +176,8 @@ __device__ __forceinline__ CurveSegment curve_segment(const float4 *cp, int i) {
 }
 
 // Whether a ray meets a curve's bounds (Curve::getAABB, primitives/curve.hpp:
-// 33-46).  A function of its own: inlined, its registers spill those of the
-// curve kernels (hair trace 3.65 -> 3.71 ms).
+// 33-46).  A function of its own: inlined, it takes registers of the curve
+// kernels (hair trace 3.65 -> 3.71 ms).
 static __device__ __noinline__ bool meets_curve(const float4 *cp, V3 o, V3 d, float tmin, float tmax) {
   const float4 a = __ldg(cp), b = __ldg(cp + 1), c = __ldg(cp + 2), e = __ldg(cp + 3);
   const float r = fmaxf(a.w, b.w);
@@ -255,10 +264,11 @@ __device__ __forceinline__ V3 moved_origin(const SceneView &S, uint32_t motion, 
 // hit in [tmin, tmax] fills `hit`.  dn points at the ray's normalised
 // direction (rectangles and spheres read it).  CURVES = false compiles the
 // curve test out (curve items then never hit), MOTION = false the moving
-// primitives.  unordered() is called for a hit of t = 0 / 0.
-template <bool CURVES, bool MOTION, class Unordered>
+// primitives.  A hit without an order is tested against the primitive's bounds
+// (EXACT, as are all tests of CURVES), or left out and the ray marked.
+template <bool CURVES, bool MOTION, bool EXACT>
 __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V3 d, const float4 *dn4, float tmin,
-                                          float tmax, HitRec &hit, float time, Unordered unordered) {
+                                          float tmax, HitRec &hit, float time, uint8_t *state) {
   Item it = load_item(S.items, idx);
   const int type = (int)f2u(it.b[3]);
   const uint32_t motion = MOTION ? f2u(it.c[3]) : 0u;
@@ -268,16 +278,14 @@ __device__ __forceinline__ bool test_item(const SceneView &S, int idx, V3 o_w, V
   if (type == ITEM_TRI) {
     h = hit_triangle(it, o, d, tmin, tmax, t, u, v);
   } else if (CURVES && type == ITEM_CURVE) {
-    h = hit_curve(S.curve_segments + 2 * PT_CURVE_SEGMENTS * (size_t)f2u(it.a[0]), o, d, tmin, tmax, t, u, v);
-    if (h && !(t <= tmax)) {  // along a segment's axis: a root of 0 / 0
-      h = meets_curve(S.curves + 4 * (size_t)__float_as_uint(__ldg(S.items[idx].a)), o, d, tmin, tmax);
-      unordered();
-    }
+    const size_t curve = f2u(it.a[0]);
+    h = hit_curve(S.curve_segments + 2 * PT_CURVE_SEGMENTS * curve, o, d, tmin, tmax, t, u, v);
+    if (h && !(t <= tmax)) h = meets_curve(S.curves + 4 * curve, o, d, tmin, tmax);
   } else if (type == ITEM_CURVE) {
     h = false;
   } else {
     const V3 dn = v3(dn4->x, dn4->y, dn4->z);
-    h = type == ITEM_QUAD ? hit_quad(it, o, dn, tmin, tmax, t, unordered) : hit_sphere(it, o, dn, tmin, tmax, t);
+    h = type == ITEM_QUAD ? hit_quad<EXACT>(it, o, dn, tmin, tmax, t, state) : hit_sphere(it, o, dn, tmin, tmax, t);
   }
   if (h) {
     hit.t = t;
@@ -310,20 +318,17 @@ __device__ __forceinline__ float slab_inv(float d) { return fabsf(d) > 1e-20f ? 
 struct WarpRays {
   float4 o[32];   // origin in the ray's current frame; w: time (motion blur)
   float4 d[32];   // direction; w: tmin
-  float4 dn[32];  // normalised direction; w: tmax of any-hit rays
+  float4 dn[32];  // normalised direction; w: tmax at the start
   int32_t leaf[64];   // leaves reached and not yet tested, oldest first ...
   uint8_t owner[64];  // ... and the lane whose ray reached each
+  uint8_t state[32];  // RayState of the lane's ray
 };
 // Closest-hit rays only: the nearest hit so far.
 struct WarpHits {
   float4 hit[32];      // t, prim (int bits, -1: none), u, v
-  uint32_t tmax[32];   // float_key of the ray's tmax; PT_TMAX_STEPS: hit.x is its tmax
-  int32_t who[32];     // tester whose hit the owner takes, else one of PT_WHO_*
-  uint32_t again;      // lanes whose rays met a hit of no order (trace_rays)
+  uint32_t tmax[32];   // float_key of the ray's tmax (RAY_ALONE: the largest key; its tmax is hit.x)
+  int32_t who[32];     // tester whose hit the owner takes
 };
-#define PT_WHO_NONE (-1)   // a closest-hit ray
-#define PT_WHO_ANY (-2)    // an any-hit ray
-#define PT_TMAX_STEPS 0xffffffffu  // of a ray that is walked leaf by leaf (and of NaN)
 // Lanes (of 32) below which a walk pauses to see whether others have ended.
 #define PT_WALK_MIN 8
 // One kernel per kind of scene: PT_BY_SCENE(S, RUN) expands RUN(CURVES, MOTION).
@@ -497,6 +502,32 @@ __device__ __forceinline__ bool visit_node(const SceneView &S, TravRay &R, TravS
   return true;
 }
 
+// The items of one leaf in order, EXACT: the result is (t, prim or -1, u, v).  A
+// function of its own, so that it lengthens no item test: with the bounds tested
+// in trace_rays' loop the 16 k-path Cornell frame's trace took 0.471 ms instead of
+// 0.452 and rough glass's 10.58 instead of 10.47 (10.44 without either).  The
+// curve kernels, which the call itself would spill (hair 3.93 ms), test the
+// bounds in the loop (3.67, from 3.57); so do any-hit rays, to which the order
+// does not matter.
+template <bool MOTION>
+static __device__ __noinline__ float4 leaf_alone(const Item *items, const float4 *motion, int32_t code, float4 o,
+                                                 float4 d, float4 dn, float tmax, bool any) {
+  SceneView S;  // what test_item reads of it
+  S.items = items;
+  S.motion = motion;
+  HitRec hit;
+  hit.t = hit.u = hit.v = 0.f;
+  hit.prim = -1;
+  const int last = (code >> 3) + (code & 7);
+  for (int i = code >> 3; i <= last; ++i) {
+    if (!test_item<false, MOTION, true>(S, i, v3(o.x, o.y, o.z), v3(d.x, d.y, d.z), &dn, d.w, tmax, hit, o.w, nullptr))
+      continue;
+    if (any) break;
+    tmax = hit.t;
+  }
+  return make_float4(hit.t, __int_as_float(hit.prim), hit.u, hit.v);
+}
+
 // Lanes of a traversal warp that hold rays: all 32 while the queue has 32
 // rays or more for every warp of the grid, else an even share of the queue.
 __device__ __forceinline__ int warp_lanes(int n) {
@@ -518,15 +549,8 @@ __device__ __forceinline__ int warp_lanes(int n) {
 // its nodes with the tmax it had when the list was last tested, i.e. it
 // may visit nodes a tighter tmax would cull, whose items then fail; its leaves
 // are tested in the order it reached them, and of two equal-t hits the later
-// one wins, as in the reference's leaf loop.
-//
-// A hit of t = NaN (0 / 0: a ray in the plane of a rectangle; rays with NaN)
-// has no order: a leaf loop accepts it, and any hit after it, whatever its
-// distance (t > tmax is false with a NaN on either side).  A closest-hit ray
-// that meets one therefore starts again and is walked leaf by leaf, each leaf
-// tested before the walk goes on, which is that loop's order to the letter.
-// What this costs the others: rough glass trace 10.41 -> 10.58 ms, Cornell 2.71
-// -> 2.76, hair 3.56 -> 3.65.
+// one wins, as in the reference's leaf loop.  (RAY_ALONE rays take a leaf off
+// the stack only when the one before is tested, with its tmax.)
 //
 // Measured against turns in which a warp either visits nodes or tests one item
 // per lane standing at a leaf (Cornell box, 256 x 256 x 64 spp): 15.3 -> 20.1
@@ -568,20 +592,17 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
   int iters = 0;
   bool active = false;     // the lane has a ray in flight
   bool pend = false;       // the list holds leaves of this lane's (last) ray
-  bool steps = false;      // its ray is walked leaf by leaf
+  bool alone = false;      // its ray is RAY_ALONE
   bool any = MODE == TRACE_ANY;
   bool exhausted = false;  // the queue has no unclaimed rays
   int qn = 0;              // leaves in the list
-  if (MODE != TRACE_ANY) {
-    if (lane == 0) H.again = 0;
-    __syncwarp();
-  }
   for (;;) {
     // ---- rays that ended: nothing left to visit or to test
     while (active && !pend && R.ref == PT_REF_EMPTY && R.sp > 0) R.ref = K.pop(R.sp);
     if (active && !pend && R.ref == PT_REF_EMPTY) {
-      if (MODE != TRACE_ANY && !steps && (H.again >> lane & 1u)) {
-        // start again, leaf by leaf
+      if (MODE != TRACE_ANY && W.state[lane] == RAY_MARKED) {
+        // again, leaf by leaf
+        W.state[lane] = RAY_ALONE;
         if (MOTION) {  // in the world's frame
           const V3 o = v3(ow[0], ow[1], ow[2]);
           W.o[lane] = make_float4(o.x, o.y, o.z, W.o[lane].w);
@@ -589,10 +610,10 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
         }
         R.tmax = W.dn[lane].w;
         H.hit[lane] = make_float4(R.tmax, __int_as_float(-1), 0.f, 0.f);
-        H.tmax[lane] = PT_TMAX_STEPS;
-        R.ref = 0;
+        H.tmax[lane] = 0xffffffffu;
+        R.ref = any ? S.any_root : 0;
         iters = 0;
-        steps = true;
+        alone = true;
       } else {
         HitRec h;
         h.prim = -1;
@@ -602,7 +623,6 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           h.prim = __float_as_int(b.y);
           h.u = b.z;
           h.v = b.w;
-          if (steps) atomicAnd(&H.again, ~(1u << lane));
         }
         done(h.prim >= 0, h);
         active = false;
@@ -627,13 +647,12 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           W.o[lane] = make_float4(o.x, o.y, o.z, time);
           W.d[lane] = make_float4(d.x, d.y, d.z, R.tmin);
           W.dn[lane] = make_float4(dn.x, dn.y, dn.z, R.tmax);
+          W.state[lane] = RAY_ORDERED;
+          alone = false;
           if (MODE != TRACE_ANY) {
-            H.hit[lane] = make_float4(R.tmax, __int_as_float(-1), 0.f, 0.f);
+            H.hit[lane] = make_float4(FLT_MAX, __int_as_float(-1), 0.f, 0.f);
             H.tmax[lane] = float_key(R.tmax);
-            H.who[lane] = any ? PT_WHO_ANY : PT_WHO_NONE;
-            // what else has no order: rays that are not finite, or so far that
-            // a product of their coordinates is not
-            steps = !(fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + xdot(d, d) < 1e18f) || R.tmax != R.tmax;
+            H.who[lane] = any ? -2 : -1;  // -2: an any-hit ray
           }
           if (MOTION) {
             ow[0] = o.x;
@@ -647,6 +666,13 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           R.sp = 0;
           iters = 0;
           active = true;
+          // rays of which every hit is without an order: not finite, or so far
+          // that products of their coordinates are not; tmax NaN
+          const float size = fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + xdot(d, d);
+          if (MODE != TRACE_ANY && (!(size < 1e18f) || R.tmax != R.tmax)) {
+            W.state[lane] = RAY_MARKED;
+            R.ref = PT_REF_EMPTY;
+          }
         }
       }
       __syncwarp();
@@ -666,7 +692,7 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
         W.owner[at] = (uint8_t)lane;
         pend = true;
         ++iters;
-        R.ref = MODE != TRACE_ANY && steps ? PT_REF_EMPTY : K.pop(R.sp);  // popped when the leaf is tested
+        R.ref = MODE != TRACE_ANY && alone ? PT_REF_EMPTY : K.pop(R.sp);  // popped when the leaf is tested
       }
       qn += __popc(lm);
       const bool ready = active && ref_is_node(R.ref) && !(MOTION && pend && ref_is_frame(R.ref));
@@ -720,20 +746,29 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
     if (lane < m) {
       const float4 o4 = W.o[own], d4 = W.d[own];
       float tm;
-      if (MODE == TRACE_MIXED) eany = H.who[own] == PT_WHO_ANY;
+      if (MODE == TRACE_MIXED) eany = H.who[own] == -2;
       if (MODE == TRACE_ANY) tm = W.dn[own].w;
-      else if (H.tmax[own] != PT_TMAX_STEPS) tm = key_float(H.tmax[own]);
-      else tm = H.hit[own].x;
+      else tm = key_float(H.tmax[own]);
       const V3 o = v3(o4.x, o4.y, o4.z), d = v3(d4.x, d4.y, d4.z);
       const int32_t code = ~lref;  // first_item << 3 | count - 1
-      const int last = (code >> 3) + (code & 7);
-      auto unordered = [&] {
-        if (MODE != TRACE_ANY && !eany) atomicOr(&H.again, 1u << own);
-      };
+      int last = (code >> 3) + (code & 7);
+      const bool again = MODE != TRACE_ANY && W.state[own] == RAY_ALONE;
+      if (again && !eany) tm = H.hit[own].x;
+      if (!CURVES && again) {
+        const float4 b = leaf_alone<MOTION>(S.items, S.motion, code, o4, d4, W.dn[own], tm, eany);
+        h.t = b.x;
+        h.prim = __float_as_int(b.y);
+        h.u = b.z;
+        h.v = b.w;
+        hit = h.prim >= 0;
+        last = -1;  // tested
+      }
       for (int i = code >> 3; i <= last; ++i) {
-        if (test_item<CURVES, MOTION>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w, unordered)) {
+        if (test_item<CURVES, MOTION, CURVES || MODE == TRACE_ANY>(S, i, o, d, &W.dn[own], d4.w, tm, h, o4.w,
+                                                                   &W.state[own])) {
           hit = true;
           if (eany) break;
+          if (CURVES && !again && !(h.t <= tm)) W.state[own] = RAY_MARKED;
           tm = h.t;
         }
       }
@@ -769,12 +804,9 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
         if (best && H.who[own] == lane) H.hit[own] = make_float4(h.t, __int_as_float(h.prim), h.u, h.v);
         __syncwarp();
         if (active && !any) {
-          R.tmax = key_float(H.tmax[lane]);
-          H.who[lane] = PT_WHO_NONE;
-          if (steps) {
-            R.tmax = H.hit[lane].x;
-            H.tmax[lane] = PT_TMAX_STEPS;
-          }
+          R.tmax = alone ? H.hit[lane].x : key_float(H.tmax[lane]);
+          if (alone) H.tmax[lane] = 0xffffffffu;
+          H.who[lane] = -1;
         }
       }
     }
