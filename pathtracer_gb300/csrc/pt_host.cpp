@@ -1778,6 +1778,7 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   V.n_nodes = (int)out.nodes.size();
   V.any_root = any_root;
   V.n_prims = n_prims;
+  V.unit_t = d->n_quads > 0 || d->n_boxes > 0 || d->n_spheres > 0;
   V.trav_cap = trav_cap > 0 ? trav_cap : PT_TRAVERSAL_CAP;
   for (int c = 0; c < 3; ++c) V.bg[c] = d->bg_color[c];
   if (d->env) {

@@ -130,6 +130,7 @@ struct SceneView {
   const float4 *motion;
   const int32_t *node_motion;  // per BVH4 node: motion index + 1 of the moving object it roots
   int32_t has_motion;
+  int32_t unit_t;    // rectangles or spheres: t along the normalised direction
   int32_t trav_cap;  // steps one ray's traversal may take before the device error flag is set
   const TexRec *textures;  // surface textures (materials' flags >> PT_MAT_TEXTURE_SHIFT)
   const float4 *prim_uv;   // per primitive texture-coordinate records (null: no textures)

@@ -329,6 +329,16 @@ struct WarpHits {
   uint32_t tmax[32];   // float_key of the ray's tmax (RAY_ALONE: the largest key; its tmax is hit.x)
   int32_t who[32];     // tester whose hit the owner takes
 };
+// A direction's squared length may be off 1 by this before the ray is walked leaf
+// by leaf in a scene with rectangles or spheres (whose t is a distance, while
+// triangles and boxes count in the direction's length).  A render's sampled
+// directions are within 1e-5.
+#define PT_UNIT_TOL 0x1p-12f
+// Nodes are culled from this much (relative) behind a hit on: the unit's part of
+// PT_UNIT_TOL, and the roundings of a node's entry and of the primitives' t, so
+// that whether a primitive that lies within them of the nearest hit is tested
+// does not depend on when that hit is found.
+#define PT_CULL_SLACK 0x1p-12f
 // Lanes (of 32) below which a walk pauses to see whether others have ended.
 #define PT_WALK_MIN 8
 // One kernel per kind of scene: PT_BY_SCENE(S, RUN) expands RUN(CURVES, MOTION).
@@ -667,9 +677,12 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
           iters = 0;
           active = true;
           // rays of which every hit is without an order: not finite, or so far
-          // that products of their coordinates are not; tmax NaN
-          const float size = fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + xdot(d, d);
-          if (MODE != TRACE_ANY && (!(size < 1e18f) || R.tmax != R.tmax)) {
+          // that products of their coordinates are not; tmax NaN; or of hits in
+          // another unit than the boxes', so that what a hit culls depends on
+          // when it is found
+          const float dd = xdot(d, d), size = fabsf(o.x) + fabsf(o.y) + fabsf(o.z) + dd;
+          if (MODE != TRACE_ANY && (!(size < 1e18f) || R.tmax != R.tmax ||
+                                    (S.unit_t && !any && fabsf(dd - 1.f) > PT_UNIT_TOL))) {
             W.state[lane] = RAY_MARKED;
             R.ref = PT_REF_EMPTY;
           }
@@ -804,7 +817,8 @@ __device__ __forceinline__ void trace_rays(const SceneView &S, int n, int *fetch
         if (best && H.who[own] == lane) H.hit[own] = make_float4(h.t, __int_as_float(h.prim), h.u, h.v);
         __syncwarp();
         if (active && !any) {
-          R.tmax = alone ? H.hit[lane].x : key_float(H.tmax[lane]);
+          const float t = key_float(H.tmax[lane]);
+          R.tmax = alone ? H.hit[lane].x : fmaf(fabsf(t), PT_CULL_SLACK, t);
           if (alone) H.tmax[lane] = 0xffffffffu;
           H.who[lane] = -1;
         }

@@ -117,3 +117,33 @@ def test_answers_do_not_depend_on_the_queue(renderer):
     t1, prim1, _ = renderer.trace_closest(sid, rays[perm])
     assert np.array_equal(prim1, prim[perm]) and np.array_equal(t1, t[perm], equal_nan=True)
     renderer.release(sid)
+
+
+@pytest.mark.parametrize("where", [0.0, 100.0])
+def test_unnormalised_directions_do_not_depend_on_the_queue(renderer, where):
+    """t is a distance on a rectangle or sphere and a multiple of the direction
+    on a triangle (and in the boxes): a ray's hit still depends on the ray alone."""
+    rng = np.random.default_rng(8)
+    sc = S.Scene()
+    mat = sc.add_material(N.LAMBERTIAN, [0.5, 0.5, 0.5])
+    for i in range(300):
+        k, a = where + rng.integers(-8, 9) * 0.25, where + rng.integers(-8, 7, 2) * 0.25
+        b = a + rng.integers(1, 12, 2) * 0.25
+        sc.add_quad(i % 3, float(k), float(a[0]), float(b[0]), float(a[1]), float(b[1]), mat)
+    for _ in range(50):
+        sc.add_sphere(tuple(where + rng.uniform(-2, 2, 3)), float(rng.uniform(0.1, 0.5)), mat)
+    sc.add_mesh(S.sphere_mesh(3, (where,) * 3, 1.5, mat, displace=0.2, seed=1))
+    sid = renderer.upload(sc)
+    n = 20011
+    o = where + rng.uniform(-4, 4, (n, 3))
+    d = (where + rng.uniform(-2, 2, (n, 3)) - o) * np.exp(rng.uniform(-3, 3, (n, 1)))
+    rays = np.concatenate([o, d], 1).astype(np.float32)
+    t, prim, _ = renderer.trace_closest(sid, rays)
+    assert (prim >= 0).mean() > 0.5
+    perm = rng.permutation(n)
+    for sel in (perm, perm[:3001], perm[:64], perm[:5]):
+        t1, prim1, _ = renderer.trace_closest(sid, rays[sel])
+        assert np.array_equal(prim1, prim[sel]) and np.array_equal(t1, t[sel])
+    hit = renderer.intersect(sid, rays[perm])
+    assert np.array_equal(hit[1], prim[perm]) and np.array_equal(hit[0], t[perm])
+    renderer.release(sid)
