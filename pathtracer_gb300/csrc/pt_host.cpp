@@ -1892,7 +1892,7 @@ Context::Context(int dev) : device(dev) {
   const char *pfb = std::getenv("PT_PAIR_FROM_BOUNCE");
   if (pfb) cfg.pair_from_bounce = std::max(0, std::atoi(pfb));
   cuda_check(cudaMalloc(&d_err, 3 * sizeof(int)), "cudaMalloc(err)");
-  d_fetch = d_err + 1;
+  fetch.counters = d_err + 1;
   cuda_check(cudaMemsetAsync(d_err, 0, 3 * sizeof(int), stream), "memset err");
   cuda_check(cudaStreamSynchronize(stream), "context init");
 }
@@ -1990,6 +1990,11 @@ const uint16_t *Context::perm_for(uint32_t seed) {
   cuda_check(cudaStreamSynchronize(stream), "upload perm");
   perms[seed] = dp;
   return dp;
+}
+
+FetchPair Context::begin_query() {
+  return fetch.begin(
+      [&](int *c) { cuda_check(cudaMemsetAsync(c, 0, 2 * sizeof(int), stream), "memset fetch counters"); });
 }
 
 Scene *Context::scene(int id) {
@@ -2607,8 +2612,9 @@ static int trace_common(void *ctx, int32_t scene_id, bool any, const float *rays
     uint8_t *docc = (uint8_t *)(buf + nn * 44);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
     if (any) cuda_check(cudaMemcpyAsync(dtm, tmaxs, nn * 4, cudaMemcpyHostToDevice, c->stream), "h2d tmax");
-    launch_trace_test(S->view, any, dr, dtm, n, tmin, tmax, dt, dp, duv, docc, c->next_fetch(), c->d_err, c->stream);
+    launch_trace_test(S->view, any, dr, dtm, n, tmin, tmax, dt, dp, duv, docc, c->begin_query(), c->d_err, c->stream);
     cuda_check(cudaGetLastError(), "trace launch");
+    c->fetch.launched();
     if (any) {
       cuda_check(cudaMemcpyAsync(occ, docc, nn, cudaMemcpyDeviceToHost, c->stream), "d2h");
     } else {
@@ -2655,8 +2661,9 @@ int pt_intersect(void *ctx, int32_t scene_id, const float *rays, int32_t n, floa
     float *dn = (float *)(buf + nn * 44);
     uint8_t *df = (uint8_t *)(buf + nn * 56);
     cuda_check(cudaMemcpyAsync(dr, rays, nn * 24, cudaMemcpyHostToDevice, c->stream), "h2d rays");
-    launch_intersect(S->view, dr, n, tmin, tmax, dt, dp, dpos, dn, df, c->next_fetch(), c->d_err, c->stream);
+    launch_intersect(S->view, dr, n, tmin, tmax, dt, dp, dpos, dn, df, c->begin_query(), c->d_err, c->stream);
     cuda_check(cudaGetLastError(), "intersect launch");
+    c->fetch.launched();
     cuda_check(cudaMemcpyAsync(t, dt, nn * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
     cuda_check(cudaMemcpyAsync(prim, dp, nn * 4, cudaMemcpyDeviceToHost, c->stream), "d2h");
     cuda_check(cudaMemcpyAsync(position, dpos, nn * 12, cudaMemcpyDeviceToHost, c->stream), "d2h");

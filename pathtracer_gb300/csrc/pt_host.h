@@ -134,14 +134,10 @@ struct Context {
   int offsets_cap = 0;
   void *d_scratch = nullptr;
   size_t scratch_cap = 0;
-  uint32_t *d_owen = nullptr;  // first digits of the Owen-scrambled dimensions (11 MB, as long as the context)
+  uint32_t *d_owen = nullptr;  // first digits of the Owen-scrambled dimensions (12 MB, as long as the context)
   int *d_err = nullptr;    // device error flag
-  int *d_fetch = nullptr;  // two fetch counters of the ray queries (behind d_err), in turn
-  int fetch_turn = 0;
-  FetchPair next_fetch() {
-    fetch_turn ^= 1;
-    return FetchPair{d_fetch + fetch_turn, d_fetch + (fetch_turn ^ 1)};
-  }
+  QueryFetch fetch;        // of the ray queries (behind d_err)
+  FetchPair begin_query();
   Profiler prof;
   Batch batch;
   int batch_wave_cap = 1 << 22;  // paths per wave of each batched job

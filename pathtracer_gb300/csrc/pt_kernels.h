@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <vector>
 #include "../../include/pathtracer_gb300.h"
+#include "pt_fetch.h"
 #include "pt_scene.cuh"
 
 #define PT_MAX_LIGHT_SAMPLES 16
@@ -130,11 +131,6 @@ struct Profiler {
     if (!on) return;
     cudaEventRecord(take(), st);
   }
-};
-
-// Fetch counters of the ray queries: this one's (0) and the next one's.
-struct FetchPair {
-  int *now, *next;
 };
 
 struct KernelInfo {
