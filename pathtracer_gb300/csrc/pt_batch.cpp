@@ -352,7 +352,7 @@ void render_batch(Context *c, const pt_job_desc *jobs, int n, float **films, pt_
     }
     G.total = M.start.back();
     G.film_floats = film_floats;
-    G.wave = (int)std::min<long long>(c->batch_wave_cap, G.total);
+    G.wave = (int)std::min<long long>(std::min(c->batch_wave_cap, wave_limit(G.ln)), G.total);
     BatchSlot &slot = B.slots[gi];
     slot.ensure(G.wave, G.ln, (int)G.members.size(), n_off, targets ? 1 : film_floats);
     std::vector<float2> offs;

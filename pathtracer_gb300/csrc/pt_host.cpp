@@ -1874,8 +1874,7 @@ Context::Context(int dev) : device(dev) {
   cfg.sort_by_material = 1;
   cfg.family_mask = 0x7f;
   const char *cap = std::getenv("PT_WAVE_PATHS");
-  // at most 2^28 - 1 paths: the shadow-ray list keeps a vertex slot in 28 bits
-  wave_cap = cap ? std::min(std::max(1024, std::atoi(cap)), (1 << PT_LIST_SHIFT) - 1) : (1 << 24);
+  wave_cap = cap ? std::max(1024, std::atoi(cap)) : (1 << 24);  // within wave_limit
   if (cap) batch_wave_cap = wave_cap;  // batched waves of the same size (tests of many-wave renders)
   // bound on one ray's traversal steps (scenes uploaded by this context);
   // exceeding it sets the device error flag, reported as PT_ERR_DEVICE
@@ -2127,10 +2126,8 @@ void Context::render_device(const pt_job_desc &j, float *d_film, pt_stats *stats
   const long long npix = (long long)j.width * j.height;
   const int e = j.spp_end ? j.spp_end : j.spp_x * j.spp_y;
   const long long total = npix * (e - j.spp_begin);
-  int n = wave_cap;
-  if (npix <= wave_cap) n = (int)((wave_cap / npix) * npix);
-  if ((long long)n > total) n = (int)total;
   const int LN = j.light_samples_x * j.light_samples_y;
+  const int n = wave_paths(npix, total, wave_cap, LN);
   ensure_queues(n, LN);
   cuda_check(cudaMemsetAsync(Q.stats, 0, 64, stream), "memset stats");
   auto t0 = std::chrono::steady_clock::now();

@@ -7,6 +7,7 @@
 #include "../../include/pathtracer_gb300.h"
 #include "pt_fetch.h"
 #include "pt_scene.cuh"
+#include "pt_wave_size.h"
 
 #define PT_MAX_LIGHT_SAMPLES 16
 #define PT_SORT_BINS 16
@@ -17,8 +18,6 @@
 #define PT_KEY_MEDIUM 9
 #define PT_FAM_MISC 7
 #define PT_HIT_MEDIUM (-2)
-// Shadow-ray list entries: the vertex slot below, the light sample above.
-#define PT_LIST_SHIFT 28
 
 namespace pt {
 
