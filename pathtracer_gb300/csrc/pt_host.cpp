@@ -1733,30 +1733,38 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   for (const Bvh4Node &N : out.nodes)
     for (int k = 0; k < 4; ++k)
       if (N.count[k] > 8) fail(PT_ERR_INVALID, "leaf of more than 8 items");
-  std::vector<void *> staged;  // freed when the scene is up
+  // What the copies to the device read lives until they are done, also when the
+  // upload ends early: declared before `freed`, which waits for them.
+  std::vector<Bvh4Node> top;
+  std::vector<PackedNode> packed;
+  std::vector<float4> curves;
+  std::vector<void *> staged;  // device memory, freed when the scene is up
   struct Freed {
     std::vector<void *> &v;
+    cudaStream_t st;
+    bool device;
     ~Freed() {
+      if (device) cudaStreamSynchronize(st);
       for (void *p : v) cudaFree(p);
     }
-  } freed{staged};
+  } freed{staged, st, device};
   int any_root = 0;
   if (device) {
     // the host tree and its hash keep the float boxes
-    const std::vector<Bvh4Node> top = any_hit_top(out, std::min(PT_TOP_UNITS, std::max(64, 4 * d->n_objects)));
+    top = any_hit_top(out, std::min(PT_TOP_UNITS, std::max(64, 4 * d->n_objects)));
     any_root = top.empty() ? 0 : (int)out.nodes.size();
     const size_t nn = out.nodes.size() + top.size();
     if (nn <= 4096) {  // packed here: two allocations on the device would take longer
-      std::vector<PackedNode> packed(nn);
+      packed.resize(nn);
       for (size_t k = 0; k < nn; ++k)
         packed[k] = pack_node(k < out.nodes.size() ? out.nodes[k] : top[k - out.nodes.size()]);
       S->nodes = up(packed);
     } else {
       const Bvh4Node *wide = dupload(out.nodes, staged, st), *wide_top = dupload(top, staged, st);
-      void *packed = nullptr;
-      cuda_check(cudaMalloc(&packed, sizeof(PackedNode) * nn), "cudaMalloc(nodes)");
-      S->owned.push_back(packed);
-      S->nodes = static_cast<PackedNode *>(packed);
+      void *nodes = nullptr;
+      cuda_check(cudaMalloc(&nodes, sizeof(PackedNode) * nn), "cudaMalloc(nodes)");
+      S->owned.push_back(nodes);
+      S->nodes = static_cast<PackedNode *>(nodes);
       launch_pack_nodes(wide, (int)out.nodes.size(), S->nodes, st);
       if (!top.empty()) launch_pack_nodes(wide_top, (int)top.size(), S->nodes + out.nodes.size(), st);
     }
@@ -1800,14 +1808,14 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
   }
   if (!prim_uv.empty()) V.prim_uv = up(prim_uv);
   if (n_curves > 0) {
-    std::vector<float4> cv(4 * (size_t)n_curves);
+    curves.resize(4 * (size_t)n_curves);
     for (int c = 0; c < n_curves; ++c) {
       const pt_curve_desc &k = d->curves[c];
       for (int j = 0; j < 4; ++j)
-        cv[4 * c + j] = make_float4(k.cps[j][0], k.cps[j][1], k.cps[j][2],
+        curves[4 * c + j] = make_float4(k.cps[j][0], k.cps[j][1], k.cps[j][2],
                                     j == 0 ? k.width0 : j == 1 ? k.width1 : 0.f);
     }
-    V.curves = up(cv);
+    V.curves = up(curves);
     if (device) {
       void *seg = nullptr;
       cuda_check(cudaMalloc(&seg, sizeof(float4) * 2 * PT_CURVE_SEGMENTS * n_curves), "cudaMalloc(curves)");
