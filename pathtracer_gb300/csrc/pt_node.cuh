@@ -19,9 +19,12 @@ static_assert(sizeof(Bvh4Node) == 128, "BVH4 node must be one 128-byte line");
 // of 256 planes per axis over the node's box, and the children's traversal
 // references.  Plane q of an axis lies at origin + (1 + q * 2^-15) * scale
 // (the bracket is a float whose middle byte is q, so it takes one byte
-// permute and no conversion).  pack_node rounds the boxes outwards, 1/8 of a
-// grid step at least, which covers the rounding of this form: a ray that
-// meets a child's box meets its packed box.
+// permute and no conversion).  pack_node rounds the boxes outwards, by 2^-20 of
+// the node's coordinates and 1/8 of a grid step at least, which covers the
+// roundings of this form and of the ray's: a ray that meets a child's box meets
+// its packed box, for origins of up to 3 times the node's coordinates or 1000
+// times its extent (each per axis).  From farther away the rounding of origin /
+// direction, 2^-24 of the origin, moves the box by more, as it moves a float box.
 //
 // Two 32-byte loads fetch it.  With float boxes a lane's visit took seven
 // 16-byte loads of a 128-byte node, one L1 wavefront per lane and load: in the
@@ -53,19 +56,27 @@ PT_HD int32_t trav_ref(int32_t child, int32_t count) {
 }
 
 // One axis of a node: `lo`, `hi` of the children (n of them), the grid and the
-// children's bytes.  The grid step is at least 2^-20 of the coordinates, so
-// that the roundings of origin (2^-25 of 2^15 steps and of the coordinates),
-// of the product with scale and of the sum stay below 1/8 of a step.
+// children's bytes.  With u = 2^-24, coordinates up to R, a ray origin o and the
+// grid's extent 2^15 steps: rounding the origin, o * inv, the fma that joins them
+// and the planes' fma moves a plane by at most u (4 R + 4 |o|), which the slack of
+// 16 u R covers for |o| <= 3 R, and by 2^-16 of the node's extent, which is far
+// below 1/8 of a step (1/2016 of the extent); so is 4 u |o| up to 1000 extents.
+// (A slack of the scene's coordinates would cover every origin in it, but a scene
+// may have a far light or a wide ground under small objects, whose boxes it
+// would swamp.)
 PT_HD void pack_axis(const float *lo, const float *hi, int n, float &origin, float &scale, uint32_t &qlo,
                      uint32_t &qhi) {
   double a = lo[0], b = hi[0];
+  bool number = true;
+  for (int c = 0; c < n; ++c) number = number && lo[c] <= hi[c];
   for (int c = 1; c < n; ++c) {
     if (lo[c] < a) a = lo[c];
     if (hi[c] > b) b = hi[c];
   }
-  const double far = fabs(a) > fabs(b) ? fabs(a) : fabs(b);
+  const double slack = (fabs(a) > fabs(b) ? fabs(a) : fabs(b)) * 0x1p-20;
+  a -= slack;
+  b += slack;
   double step = (b - a) / 252.0;
-  if (step < far * 0x1p-20) step = far * 0x1p-20;
   if (step < 1e-30) step = 1e-30;
   scale = (float)(step * 32768.0);
   step = (double)scale / 32768.0;
@@ -74,11 +85,14 @@ PT_HD void pack_axis(const float *lo, const float *hi, int n, float &origin, flo
   qlo = 0xffffffffu;  // empty slots: inverted
   qhi = 0;
   for (int c = 0; c < n; ++c) {
-    const double l = floor((lo[c] - zero) / step - 0.125), h = ceil((hi[c] - zero) / step + 0.125);
-    const uint32_t ql = l < 0.0 ? 0u : (uint32_t)l, qh = h > 255.0 ? 255u : (uint32_t)h;
+    const double l = floor((lo[c] - slack - zero) / step - 0.125), h = ceil((hi[c] + slack - zero) / step + 0.125);
+    const uint32_t ql = l >= 0.0 ? (uint32_t)l : 0u, qh = h <= 255.0 ? (uint32_t)h : 255u;
     qlo = (qlo & ~(255u << (8 * c))) | (ql << (8 * c));
     qhi |= qh << (8 * c);
   }
+  // a bound that is not a number: planes that are none either, which the slab
+  // test's min / max drop, as they drop such a float bound
+  if (!number) origin = scale = NAN;
 }
 PT_HD PackedNode pack_node(const Bvh4Node &N) {
   PackedNode P;
