@@ -249,6 +249,8 @@ PT_HD uint64_t path_key(uint32_t seed, uint64_t sample_id) {
 // table's entries.
 #define PT_OWEN_DIMS 64
 #define PT_OWEN_ENTRIES (1u << 17)
+// Owen-scrambled digits are tested for being settled from this power of the base on.
+#define PT_OWEN_SETTLED (1ull << 35)
 struct HaltonTables {
   int32_t prime[PT_PRIME_COUNT];
   int32_t ndigits[PT_PRIME_COUNT];    // digits visited by the double loop test
@@ -259,7 +261,7 @@ struct HaltonTables {
   uint32_t div_magic[PT_PRIME_COUNT];
   int32_t div_shift[PT_PRIME_COUNT];  // shift; bit 6 set: the 33-bit (add) form
   // Owen-scrambled digits after which the value is tested for being settled
-  // (the least k with prime^k >= 2^35), and prime^(ndigits - owen_check)
+  // (the least k with prime^k >= PT_OWEN_SETTLED), and prime^(ndigits - owen_check)
   int32_t owen_check[PT_PRIME_COUNT];
   uint64_t owen_tail[PT_PRIME_COUNT];
   // Tables of the first Owen-scrambled digits (owen_radical_inverse): the
@@ -407,7 +409,7 @@ PT_HD void owen_digit(const HaltonTables &T, int bi, uint32_t base, uint32_t w, 
 // The scrambled digits of the first T.owen_first digits depend on the index
 // modulo T.owen_pow only: `first`, the dimension's table by that remainder (or
 // null), gives them with one load in place of 2 (base 97) to 17 (base 2) of the
-// 6 to 38 digits up to the early end.
+// 6 to 35 digits up to the early end.
 template <int C>
 PT_HD float owen_digits(const HaltonTables &T, int bi, uint32_t hash, uint32_t index, const uint32_t *first) {
   const uint32_t base = (uint32_t)T.prime[bi];
@@ -471,6 +473,39 @@ inline uint32_t owen_table_layout(HaltonTables &T) {
   T.owen_at[0] = 0;
   for (int d = 0; d < PT_OWEN_DIMS; ++d) T.owen_at[d + 1] = T.owen_at[d] + T.owen_pow[d % PT_PRIME_COUNT];
   return T.owen_at[PT_OWEN_DIMS];
+}
+// gl::Primes (utility.hpp:400-402), digit counts and inverse radix powers
+// exactly as the double loop of owenScrambledRadicalInverse computes them
+// (digitPerm.hpp:105-128).
+inline HaltonTables make_halton_tables() {
+  static const int primes[PT_PRIME_COUNT] = {2,  3,  5,  7,  11, 13, 17, 19, 23, 29, 31, 37, 41,
+                                             43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97};
+  HaltonTables T;
+  int off = 0;
+  for (int b = 0; b < PT_PRIME_COUNT; ++b) {
+    const int base = primes[b];
+    T.prime[b] = base;
+    const double inv_base = 1.0 / (double)base;
+    double inv_base_m = 1.0;
+    int nd = 0;
+    while (1.0 - (base - 1) * inv_base_m < 1.0) {
+      ++nd;
+      inv_base_m *= inv_base;
+    }
+    T.ndigits[b] = nd;
+    T.inv_base_m[b] = inv_base_m;
+    T.perm_offset[b] = off;
+    off += nd * base;
+    div_invariant((uint32_t)base, T.div_magic[b], T.div_shift[b]);
+    int check = 0;
+    for (uint64_t p = 1; p < PT_OWEN_SETTLED && check < nd; p *= (uint64_t)base) ++check;
+    uint64_t tail = 1;
+    for (int r = check; r < nd; ++r) tail *= (uint64_t)base;
+    T.owen_check[b] = check;
+    T.owen_tail[b] = tail;
+  }
+  owen_table_layout(T);
+  return T;
 }
 
 // gl::scrambledRadicalInverse with DigitPermutation tables

@@ -34,41 +34,6 @@ void cuda_check(cudaError_t e, const char *what) {
   if (e != cudaSuccess) fail(PT_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// ------------------------------------------------------- Halton tables
-// gl::Primes (utility.hpp:400-402), digit counts and inverse radix powers
-// exactly as the double loop of owenScrambledRadicalInverse computes them
-// (digitPerm.hpp:105-128).
-HaltonTables make_halton_tables() {
-  static const int primes[PT_PRIME_COUNT] = {2,  3,  5,  7,  11, 13, 17, 19, 23, 29, 31, 37, 41,
-                                             43, 47, 53, 59, 61, 67, 71, 73, 79, 83, 89, 97};
-  HaltonTables T;
-  int off = 0;
-  for (int b = 0; b < PT_PRIME_COUNT; ++b) {
-    const int base = primes[b];
-    T.prime[b] = base;
-    const double inv_base = 1.0 / (double)base;
-    double inv_base_m = 1.0;
-    int nd = 0;
-    while (1.0 - (base - 1) * inv_base_m < 1.0) {
-      ++nd;
-      inv_base_m *= inv_base;
-    }
-    T.ndigits[b] = nd;
-    T.inv_base_m[b] = inv_base_m;
-    T.perm_offset[b] = off;
-    off += nd * base;
-    div_invariant((uint32_t)base, T.div_magic[b], T.div_shift[b]);
-    int check = 0;
-    for (uint64_t p = 1; p < (1ull << 35) && check < nd; p *= (uint64_t)base) ++check;
-    uint64_t tail = 1;
-    for (int r = check; r < nd; ++r) tail *= (uint64_t)base;
-    T.owen_check[b] = check;
-    T.owen_tail[b] = tail;
-  }
-  owen_table_layout(T);
-  return T;
-}
-
 // MurmurHash64A (Austin Appleby, public domain), the byte hash that
 // pbrt::hash applies to its packed arguments (hash.hpp:10-58, 84-91).
 static uint64_t murmur64a(const unsigned char *key, size_t len, uint64_t seed) {

@@ -22,7 +22,6 @@ struct PtError : std::runtime_error {
 [[noreturn]] void fail(int code, const std::string &msg);
 void cuda_check(cudaError_t e, const char *what);
 
-HaltonTables make_halton_tables();
 std::vector<uint16_t> make_digit_permutations(const HaltonTables &T, uint32_t seed);
 MatRec derive_material(const pt_material_desc &m);
 CameraView make_camera(const pt_camera_desc &c);
