@@ -787,7 +787,7 @@ def run_ours(args, rank, world, local_rank):
         "config": {"workload": wl["desc"], "step": f"{k} spp x {W}x{H} px = {W * H * k} paths",
                    "estimator": wl["est_name"], "triangles": info["triangles"], "bvh4_nodes": info["bvh4_nodes"],
                    "bvh": "BVH4 collapsed from the reference's own trees (the library default)",
-                   "l2": "inputs larger than L2: BVH + leaves "
+                   "l2": "inputs larger than L2: flattened scene (nodes as built, 128 B) "
                          f"{info['device_bytes'] / 1e6:.0f} MB and ~{tot['bytes'] / args.steps / 1e9:.1f} GB of "
                          "queue traffic per step (L2 129 MB)",
                    "parallelism": f"replicas x{world} (sample ranges per rank)"},

@@ -381,8 +381,10 @@ int pt_load_image(const char *path, int32_t flip_y, int32_t is_hdr, float **texe
                   int32_t *height);
 int pt_free_image(float *texels);
 /* Counts of the flattened scene: [0] triangles, [1] quads, [2] spheres,
- * [3] BVH4 nodes, [4] lights, [5] bytes of the flattened scene (its BVH4 nodes
- * counted at 128 bytes as built; the device keeps them packed to 64). */
+ * [3] BVH4 nodes, [4] lights, [5] bytes of the flattened scene: nodes at 128
+ * bytes as built, leaf items, shading records, materials, lights and the
+ * environment.  The device keeps the nodes packed to 64 bytes and, not counted
+ * here, the any-hit rays' top, curve segments and textures. */
 int pt_scene_info(void *ctx, int32_t scene_id, int64_t *out6);
 
 /* Renders one job synchronously (replaces the pixel loop of

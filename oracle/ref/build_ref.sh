@@ -1,6 +1,6 @@
 #!/usr/bin/env bash
 # Builds oracle/_ref/libref_harness.so from the reference sources where they
-# lie (default /root/reference; override with REF_ROOT).  Oracle
+# lie (REF_ROOT, else the default below).  Oracle
 # infrastructure: used only to pin the CPU restatement and to generate the
 # golden fixtures in tests/golden/.  The reference's own CMake build is not
 # used; the flags below restate src/CMakeLists.txt:19-22 (BIASED_SAMPLING),

@@ -1719,7 +1719,10 @@ std::unique_ptr<Scene> build_scene(const pt_scene_desc *d_in, cudaStream_t st, b
     top = any_hit_top(out, std::min(PT_TOP_UNITS, std::max(64, 4 * d->n_objects)));
     any_root = top.empty() ? 0 : (int)out.nodes.size();
     const size_t nn = out.nodes.size() + top.size();
-    if (nn <= 4096) {  // packed here: two allocations on the device would take longer
+    // Few nodes are packed here: two allocations on the device take longer.  48
+    // nodes: an upload of 279 us against 326; 451: 2.10 ms either way; 2869: 11.6
+    // against 11.5.
+    if (nn <= 4096) {
       packed.resize(nn);
       for (size_t k = 0; k < nn; ++k)
         packed[k] = pack_node(k < out.nodes.size() ? out.nodes[k] : top[k - out.nodes.size()]);

@@ -3,10 +3,10 @@
 // The BVH4 is collapsed from the reference's own binary trees (top level
 // BVHNode, bvh.hpp:46-102; per mesh MeshBVHNode, meshBVH.cpp:6-55), so the
 // leaves hold exactly the reference's leaf primitive sets.  Closest-hit
-// traversal is near-to-far; the per-thread stacks are in SHARED memory
-// (column per thread, bank-conflict free).  Primitive tests restate the reference arithmetic
-// with rounded, never-fused operations so that hit distances match the
-// reference bit for bit:
+// traversal is near-to-far; the first PT_STACK_SHARED entries of a thread's stack
+// are in shared memory (column per thread, bank-conflict free), the others in
+// local memory.  Primitive tests restate the reference arithmetic with rounded,
+// never-fused operations so that hit distances match the reference bit for bit:
 //   triangle  MeshBVHNode::hitTriangle  meshBVH.cpp:85-143
 //   rectangle AARectangle<axis>::intersect  primitive.cpp:31-122
 //   sphere    Sphere::intersect  primitive.hpp:124-170
@@ -129,8 +129,7 @@ __device__ __forceinline__ void ld32b(const void *p, uint32_t *v) {
       : "l"(p));
 }
 
-// Cubic Bezier point and derivative (primitives/bezier.hpp:10-36).
-// Bezier point with every operation separately rounded (never fused), in
+// Cubic Bezier point, every operation separately rounded (never fused) in
 // bezier.hpp:10-18's order, so that curve hits round like the reference's.
 __device__ __forceinline__ V3 bezier_point(const float4 *cp, float u) {
   const float u1 = xsub(1.0f, u);
@@ -142,6 +141,7 @@ __device__ __forceinline__ V3 bezier_point(const float4 *cp, float u) {
   };
   return v3(comb(c0.x, c1.x, c2.x, c3.x), comb(c0.y, c1.y, c2.y, c3.y), comb(c0.z, c1.z, c2.z, c3.z));
 }
+// Its derivative (bezier.hpp:20-36).
 __device__ __forceinline__ V3 bezier_tangent(const float4 *cp, float u) {
   const float4 c0 = __ldg(cp), c1 = __ldg(cp + 1), c2 = __ldg(cp + 2), c3 = __ldg(cp + 3);
   const V3 d0 = 3.0f * (v3(c1.x, c1.y, c1.z) - v3(c0.x, c0.y, c0.z));

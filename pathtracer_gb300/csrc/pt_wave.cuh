@@ -386,15 +386,6 @@ __global__ void __launch_bounds__(128, CURVES ? 7 : 8) k_trace_closest(SceneView
   trace_closest_body<MJ, CURVES, MOTION>(S, J, T, Q, qsel, bounce, g0, smem);
 }
 
-// k_trace_pair: the closest-hit rays of bounce `bounce` (RayQueue qsel)
-// and the shadow rays of the bounce before it (ShadowQueue) in ONE persistent launch.  Both queues come from the
-// same shade pass and neither reads the other's output, so one index space
-// [0, n_closest + n_shadow) is fetched with one counter (Q.counts[4]):
-// closest rays first (the sort and shade passes wait on them), then shadow
-// rays.  A bounce then has one sparse tail instead of two.  Per ray the work
-// is exactly k_trace_closest's or k_trace_shadow's, so results are the same;
-// the shadow terms are still added (k_shadow_resolve) before the next shade
-// pass, in the same order.
 // Shadow ray r of the list; returns its ShadowQueue slot.
 __device__ __forceinline__ size_t fetch_shadow(const SceneView &S, const Queues &Q, int r, V3 &o, V3 &d, float &tmin,
                                                float &tmax, float &time) {
@@ -409,6 +400,15 @@ __device__ __forceinline__ size_t fetch_shadow(const SceneView &S, const Queues 
   tmax = dd.w;
   return slot;
 }
+// k_trace_pair: the closest-hit rays of bounce `bounce` (RayQueue qsel) and the
+// shadow rays of the bounce before it (ShadowQueue) in ONE persistent launch.  Both
+// queues come from the same shade pass and neither reads the other's output, so
+// one index space [0, n_closest + n_shadow) is fetched with one counter
+// (Q.counts[4]): closest rays first (the sort and shade passes wait on them), then
+// shadow rays.  A bounce then has one sparse tail instead of two.  Per ray the work
+// is k_trace_closest's or k_trace_shadow's, so results are the same; the shadow
+// terms are still added (k_shadow_resolve) before the next shade pass, in the same
+// order.
 template <bool MJ, bool CURVES, bool MOTION>
 __device__ __forceinline__ void trace_pair_body(const SceneView &S, const DeviceJob &J, const JobTable &T,
                                                 const Queues &Q, int qsel, int bounce, long long g0, char *smem) {

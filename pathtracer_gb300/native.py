@@ -437,6 +437,8 @@ class Renderer:
                 "build_us": out[4]}
 
     def scene_info(self, sid: int):
+        """pt_scene_info: counts of the flattened scene, and its bytes with the
+        nodes as built (`device_bytes`; the device packs them to half)."""
         out = (C.c_int64 * 6)()
         self._check(self.lib.pt_scene_info(self.ctx, sid, out))
         return dict(zip(["triangles", "quads", "spheres", "bvh4_nodes", "lights", "device_bytes"], list(out)))
