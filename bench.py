@@ -58,7 +58,7 @@ FALLBACK_HBM_GBS = 6800.0
 # traversal-stage launches (closest, paired, shadow and the shadow resolve) of
 # one step of 16 spp of every pixel, per (workload, estimator); from a
 # one-pass ncu capture of the same bench command
-NCU_TRAVERSAL_BYTES_PER_STEP = {("rough_glass", 0): 7.151e9}
+NCU_TRAVERSAL_BYTES_PER_STEP = {("rough_glass", 0): 7.156e9}
 # Algorithmic queue bytes per unit, by stage: the records each stage must
 # read or write in this layout -- 192 B per path vertex,
 # 88 B per shadow ray (44 written by shade, 44 read by the traversal) and FP32
